@@ -43,7 +43,7 @@ struct Batch {
     long long n_tasks = 0;
     unsigned long long* d_queue = nullptr;
     int* d_error = nullptr;
-    RayResult* d_ray_res = nullptr;
+    void* d_rays = nullptr;
     size_t ray_cap = 0;
     Tuning tuning;
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
@@ -92,10 +92,10 @@ int build(Batch* b) {
     b->n_tasks = begin;
     const size_t need = (size_t)std::min<long long>(std::max<long long>(begin, 1), kBatchRoundTasks) * kTaskRays;
     if (need > b->ray_cap) {
-        cudaFree(b->d_ray_res);
-        b->d_ray_res = nullptr;
+        cudaFree(b->d_rays);
+        b->d_rays = nullptr;
         b->ray_cap = 0;
-        LUMRAD_TRY(cudaMalloc(&b->d_ray_res, need * sizeof(RayResult)));
+        LUMRAD_TRY(cudaMalloc(&b->d_rays, need * kRayBytes));
         b->ray_cap = need;
     }
     b->release_graphs();
@@ -107,7 +107,7 @@ int build(Batch* b) {
         la.n_tasks = b->n_tasks;
         la.queue = b->d_queue;
         la.error = b->d_error;
-        la.ray_res = b->d_ray_res;
+        la.rays = ray_buffer(b->d_rays, b->ray_cap);
         la.round_tasks = kBatchRoundTasks;
         la.in_cta = combines_in_cta(b->h_table[k], nw) ? 1 : 0;
         la.guided_div = b->tuning.guided_div;
@@ -250,7 +250,7 @@ void lumrad_batch_destroy(LumRadBatch batch) {
     }
     cudaFree(b->d_queue);
     cudaFree(b->d_error);
-    cudaFree(b->d_ray_res);
+    cudaFree(b->d_rays);
     if (b->ev_start) cudaEventDestroy(b->ev_start);
     if (b->ev_end) cudaEventDestroy(b->ev_end);
     if (b->stream) cudaStreamDestroy(b->stream);

@@ -115,7 +115,7 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
     if (rc) return rc;
 
     // page-locked staging (see Context::h_blk), made on the first call
-    const size_t off_cgrid = w.W * sizeof(int16_t), off_cslot = off_cgrid + w.W * sizeof(uint16_t);
+    const size_t off_cgrid = w.W * sizeof(int16_t), off_cslot = off_cgrid + (compact_cells(w.X, w.Y, w.Z) * sizeof(uint16_t) + 15) / 16 * 16;
     const size_t n_cslot = (size_t)w.n_slots + 128;
     const size_t off_copies = off_cslot + n_cslot * sizeof(int);
     if (!c->h_blk) {
@@ -240,7 +240,7 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
         LUMRAD_TRY(cudaMalloc(&w.d_cslot, cap * sizeof(int)));
         w.cbits_cap = cap;
     }
-    // the compact grid and slots through the staging area (both fit: at most W uint16 ids, and
+    // the compact grid and slots through the staging area (both fit: uint16 ids at most, and
     // at most n_slots + 66 compact ids)
     const void* cslot_src = w.h_cslot.data();
     if (w.h_cslot.size() <= n_cslot) {

@@ -8,7 +8,7 @@
 //
 // Device layout of a world (all resident between passes):
 //   grid      int16  X*Y*Z            block ids, x-fastest
-//   cgrid     uint8 / uint16 X*Y*Z    compact ids (0 = air), rebuilt when the grid or palette changes
+//   cgrid     uint8 / uint16 (X+1)*(Y+1)*(Z+1)   compact ids (0 = air), rebuilt when the grid or palette changes
 //   cbits     uint32 128 per compact id   voxel occupancy of each compact id
 //   pal       uint8  slots*4096       voxel values, voxel (x,y,z) at x + 16y + 256z
 //   mats      float4 256              (r, g, b, emission)
@@ -66,7 +66,7 @@ int DeviceWorld::init(int X_, int Y_, int Z_, int slots, int precision_, cudaStr
     h_mats.assign(LUMRAD_MATERIALS, LumRadMaterial{});
     h_mats_dev.assign(LUMRAD_MATERIALS, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
     LUMRAD_TRY(cudaMalloc(&d_grid, W * sizeof(int16_t)));
-    LUMRAD_TRY(cudaMalloc(&d_cgrid, W * sizeof(uint16_t)));
+    LUMRAD_TRY(cudaMalloc(&d_cgrid, compact_cells(X, Y, Z) * sizeof(uint16_t)));
     LUMRAD_TRY(cudaMalloc(&d_pal, h_pal.size()));
     LUMRAD_TRY(cudaMalloc(&d_mats, LUMRAD_MATERIALS * sizeof(float4)));
     LUMRAD_TRY(cudaMalloc(&d_stats, 2 * sizeof(unsigned long long)));
@@ -108,7 +108,7 @@ int DeviceWorld::evict(cudaStream_t stream) {
 int DeviceWorld::readmit(cudaStream_t stream) {
     if (!evicted) return LUMRAD_OK;
     LUMRAD_TRY(cudaMalloc(&d_grid, W * sizeof(int16_t)));
-    LUMRAD_TRY(cudaMalloc(&d_cgrid, W * sizeof(uint16_t)));
+    LUMRAD_TRY(cudaMalloc(&d_cgrid, compact_cells(X, Y, Z) * sizeof(uint16_t)));
     LUMRAD_TRY(cudaMalloc(&d_pal, h_pal_dev.size()));
     LUMRAD_TRY(cudaMalloc(&d_mats, LUMRAD_MATERIALS * sizeof(float4)));
     LUMRAD_TRY(cudaMalloc(&d_stats, 2 * sizeof(unsigned long long)));
@@ -150,12 +150,19 @@ void DeviceWorld::build_compact(const int16_t* g, bool host_bits) {
         if (id_to_c[(uint16_t)g[i]] >= 0) continue;
         if (compact_of(g[i], &assigned) < 0) cgrid_wide = true;   // > 256 ids: uint16
     }
-    h_cgrid.resize(W * (cgrid_wide ? 2 : 1));
-    for (size_t i = 0; i < W; i++) {
-        const int32_t c = id_to_c[(uint16_t)g[i]];
-        if (cgrid_wide) reinterpret_cast<uint16_t*>(h_cgrid.data())[i] = (uint16_t)c;
-        else h_cgrid[i] = (uint8_t)c;
-    }
+    h_cgrid.assign(compact_cells(X, Y, Z) * (cgrid_wide ? 2 : 1), 0);   // the cells past the grid: block 0
+    for (int z = 0; z < Z; z++)
+        for (int y = 0; y < Y; y++) {
+            const int16_t* row = g + (size_t)X * ((size_t)y + (size_t)Y * z);
+            const size_t o = (size_t)(X + 1) * ((size_t)y + (size_t)(Y + 1) * z);
+            if (cgrid_wide) {
+                uint16_t* out = reinterpret_cast<uint16_t*>(h_cgrid.data()) + o;
+                for (int x = 0; x < X; x++) out[x] = (uint16_t)id_to_c[(uint16_t)row[x]];
+            } else {
+                uint8_t* out = h_cgrid.data() + o;
+                for (int x = 0; x < X; x++) out[x] = (uint8_t)id_to_c[(uint16_t)row[x]];
+            }
+        }
     skip_host_bits = false;
 }
 
@@ -185,7 +192,7 @@ int DeviceWorld::compact_of(int16_t b, bool* assigned) {
 }
 
 size_t DeviceWorld::footprint() const {
-    size_t b = W * sizeof(int16_t) + W * sizeof(uint16_t) + cbits_cap * (128 * sizeof(uint32_t) + sizeof(int)) + h_pal.size() +
+    size_t b = W * sizeof(int16_t) + compact_cells(X, Y, Z) * sizeof(uint16_t) + cbits_cap * (128 * sizeof(uint32_t) + sizeof(int)) + h_pal.size() +
                LUMRAD_MATERIALS * sizeof(float4) + 2 * W * rad_stride + scratch_cap * sizeof(float4) +
                count_cap * sizeof(int) + 2 * sizeof(unsigned long long) + hits_cap * sizeof(LumRadHit);
     for (auto& kv : d_dirs) b += (size_t)kv.first * sizeof(float4);
@@ -369,15 +376,15 @@ int Context::ensure_rays(long long n_tasks, long long cap_tasks) {
     const size_t need = (size_t)std::min<long long>(std::max<long long>(n_tasks, 1), cap_tasks) * kTaskRays;
     if (need <= ray_cap) return LUMRAD_OK;
     LUMRAD_TRY(cudaStreamSynchronize(stream));
-    cudaFree(d_ray_res);
-    cudaFree(d_ray_res2);
+    for (void*& r : d_rays) {
+        cudaFree(r);
+        r = nullptr;
+    }
     cudaFree(d_ray_blk);
-    d_ray_res = d_ray_res2 = nullptr;
     d_ray_blk = nullptr;
     ray_cap = 0;
     pass_mark = -1;   // the buffers are new: no launch overlaps the synchronised one
-    LUMRAD_TRY(cudaMalloc(&d_ray_res, need * sizeof(RayResult)));
-    LUMRAD_TRY(cudaMalloc(&d_ray_res2, need * sizeof(RayResult)));
+    for (void*& r : d_rays) LUMRAD_TRY(cudaMalloc(&r, need * kRayBytes));
     LUMRAD_TRY(cudaMalloc(&d_ray_blk, need * sizeof(int)));
     ray_cap = need;
     return LUMRAD_OK;
@@ -456,7 +463,7 @@ int Context::run_pass(const short4* d_reqs, int n, const LumRadPassParams* p_in,
     // the march may start in the previous pass's finalize tail: see pass_mark (the list must not
     // come from a kernel, the hits use the one record buffer)
     const bool dependent = !p.record_hits && !dev_count && pass_mark == api_calls - 1 && uploads_mark == world.uploads;
-    la.ray_res = ray_side ? d_ray_res2 : d_ray_res;
+    la.rays = ray_buffer(d_rays[ray_side], ray_cap);
     ray_side ^= 1;
     la.ray_blk = d_ray_blk;
     la.dev_count = dev_count;
@@ -568,7 +575,7 @@ int Context::run_passes(const short4* const* reqs, const int* ns, const LumRadPa
             la.queue = d_queue;
             la.error = d_error;
             if ((rc = ensure_rays(la.n_tasks))) return rc;
-            la.ray_res = side ? d_ray_res2 : d_ray_res;
+            la.rays = ray_buffer(d_rays[side], ray_cap);
             la.ray_blk = d_ray_blk;
             LUMRAD_TRY(launch_radiance(la, world.precision, false, num_sms, stream, dependent));
             dependent = false;
@@ -620,7 +627,7 @@ int Context::run_passes(const short4* const* reqs, const int* ns, const LumRadPa
         la.n_tasks = total;
         la.queue = d_queue;
         la.error = d_error;
-        la.ray_res = side ? d_ray_res2 : d_ray_res;
+        la.rays = ray_buffer(d_rays[side], ray_cap);
         la.ray_blk = d_ray_blk;
         la.pass_mask = side ? d_pass_mask2 : d_pass_mask;
         if (first) la.clear_stats = world.d_stats;
@@ -708,8 +715,7 @@ void Context::release() {
     cudaFree(d_req);
     cudaFree(d_queue);
     cudaFree(d_error);
-    cudaFree(d_ray_res);
-    cudaFree(d_ray_res2);
+    for (void* r : d_rays) cudaFree(r);
     cudaFree(d_ray_blk);
     for (int h = 0; h < 2; h++) {
         if (h_ptab[h]) cudaFreeHost(h_ptab[h]);

@@ -30,18 +30,31 @@ constexpr int kMultiPasses = 32;
 // until the passes' finalize launches: 2^19 tasks = 537 MB)
 constexpr int kMultiTasks = 1 << 19;
 
-// A marched ray as the march leaves it for the finalize (32 B, two 16-byte words): the coarse
-// fraction's bits and the info word (bits 0-15 coarse steps, 16-23 coarse voxel (records only),
-// 24 hit, 25 stopped by the step bound), then the ray's origin and direction as the march set them
-// up.  The finalize reads the ray back instead of setting it up again: against 8-byte results and
-// a second set-up, the march +2.8% (four times the bytes stored) and each finalize -8.5%; the
-// 8-pass step -3.0%, a single pass -2.4%, a batch -1.9% (bit-identical).
-struct __align__(16) RayResult {
-    uint32_t frac, info;
-    float ox, oy;
-    float oz, dx, dy, dz;
+// A ray's bytes between the march and the finalize, in three arrays over the rays of a launch's
+// buffer (RayBuffer): origin and direction x (16 B), direction y and z (8 B), both written by the
+// set-up, one task's 32 rays side by side; and the result (8 B): the coarse fraction's bits and
+// the info word (bits 0-15 coarse steps, 16-23 coarse voxel (records only), 24 hit, 25 stopped by
+// the step bound), written when the ray ends.  The finalize reads the ray back instead of setting
+// it up again.  (Rays end a few lanes at a time: one 32-byte record per ending ray took the march's
+// loop two 16-byte stores and their register moves per iteration where the set-up's whole-warp
+// stores are two per task.)
+constexpr size_t kRayBytes = 32;
+struct RayBuffer {
+    float4* od;                  // ox, oy, oz, dx
+    float2* dd;                  // dy, dz
+    uint2* res;                  // fraction bits, info
 };
-static_assert(sizeof(RayResult) == 32, "two 16-byte words");
+// the arrays of a buffer of kRayBytes * cap bytes (cap: its rays, a multiple of 32)
+inline RayBuffer ray_buffer(void* base, size_t cap) {
+    char* p = static_cast<char*>(base);
+    return RayBuffer{reinterpret_cast<float4*>(p), reinterpret_cast<float2*>(p + 16 * cap),
+                     reinterpret_cast<uint2*>(p + 24 * cap)};
+}
+
+// Cells of a world's compact grid: one more than the grid on the high side of each axis, all of
+// block 0 (what a lookup past the grid reads), so that the march reads the cell a ray leaves the
+// world through without testing the grid's range.
+inline size_t compact_cells(int X, int Y, int Z) { return (size_t)(X + 1) * (Y + 1) * (Z + 1); }
 
 // One world's pass as the kernels see it (all pointers are device pointers).
 //
@@ -53,7 +66,7 @@ static_assert(sizeof(RayResult) == 32, "two 16-byte words");
 struct WorldPass {
     int X, Y, Z;                 // blocks per axis
     int cgrid_wide;              // 0: uint8 compact ids, 1: uint16
-    const void* cgrid;           // X*Y*Z compact ids, x-fastest
+    const void* cgrid;           // (X+1)*(Y+1)*(Z+1) compact ids, x-fastest; 0 past the grid (compact_cells)
     const uint32_t* cbits;       // 128 words per compact id
     const int* cslot;            // palette slot of each compact id (-1: none), or null: read the grid
     const int16_t* grid;         // X*Y*Z block ids
@@ -90,10 +103,10 @@ struct LaunchArgs {
     long long n_tasks;           // tasks of all worlds
     unsigned long long* queue;   // kQueueWords words (see kQueueWords); zero between launches
     int* error;                  // set non-zero if a warp's scheduler stops making progress
-    RayResult* ray_res;          // per ray of the round
+    RayBuffer rays;              // per ray of the round
     int* ray_blk;                // per ray of the round: block id at the last coarse step (records)
-    int ray_origin;              // task whose rays start ray_res (the march launch's chunk_begin)
-    int round_tasks;             // tasks per march/finalize round (0: kChunkTasks); ray_res holds one round
+    int ray_origin;              // task whose rays start the buffer (the march launch's chunk_begin)
+    int round_tasks;             // tasks per march/finalize round (0: kChunkTasks); the ray buffer holds one round
     int in_cta;                  // table launches: 1 if combines_in_cta holds for every world (the lean
                                  // finalize kernel), 0 for the general one
     int force_lean;              // test hook: the lean finalize kernel even where a probe's subgroups span

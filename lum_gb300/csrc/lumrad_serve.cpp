@@ -143,7 +143,7 @@ struct Slot {
     unsigned long long* d_queue = nullptr;
     int* d_error = nullptr;
     int* h_error = nullptr;       // pinned
-    RayResult* d_ray_res = nullptr;
+    void* d_rays = nullptr;
     bool busy = false;
     std::vector<SRequest> reqs;
     std::vector<int> probes;
@@ -460,7 +460,7 @@ int launch(Server* sv, int k, int free_slots, bool* started) {
     la.n_tasks = begin;
     la.queue = sl.d_queue;
     la.error = sl.d_error;
-    la.ray_res = sl.d_ray_res;
+    la.rays = ray_buffer(sl.d_rays, (size_t)kChunkTasks * kTaskRays);
     la.in_cta = combines_in_cta(table, nl) ? 1 : 0;
     la.guided_div = sv->tuning.guided_div;
     la.max_chunk = sv->tuning.max_chunk;
@@ -547,7 +547,7 @@ struct DevLane {
     long long chunk_cap = 0, chunks_total = 0;
     int* d_error = nullptr;
     unsigned long long* d_queue = nullptr;
-    RayResult* d_ray_res = nullptr;
+    void* d_rays = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_end = nullptr;
     cudaGraph_t graph = nullptr;
@@ -588,7 +588,7 @@ int devloop_lane_create(Server* sv, DevLoopHost& dl, DevLane& ln) {
     LUMRAD_TRY(cudaMalloc(&ln.d_loop, sizeof(DevLoop)));
     LUMRAD_TRY(cudaMalloc(&ln.d_error, sizeof(int)));
     LUMRAD_TRY(cudaMalloc(&ln.d_queue, kQueueWords * sizeof(unsigned long long)));
-    LUMRAD_TRY(cudaMalloc(&ln.d_ray_res, (size_t)dl.max_tasks * kTaskRays * sizeof(RayResult)));
+    LUMRAD_TRY(cudaMalloc(&ln.d_rays, (size_t)dl.max_tasks * kTaskRays * kRayBytes));
     LUMRAD_TRY(cudaMemsetAsync(ln.d_error, 0, sizeof(int), ln.stream));
     LUMRAD_TRY(cudaMemsetAsync(ln.d_queue, 0, kQueueWords * sizeof(unsigned long long), ln.stream));
     std::unique_ptr<DevLoop> h(new DevLoop());
@@ -639,7 +639,7 @@ int devloop_lane_create(Server* sv, DevLoopHost& dl, DevLane& ln) {
     la.n_tasks = dl.max_tasks;
     la.queue = ln.d_queue;
     la.error = ln.d_error;
-    la.ray_res = ln.d_ray_res;
+    la.rays = ray_buffer(ln.d_rays, (size_t)dl.max_tasks * kTaskRays);
     la.in_cta = 1;
     LUMRAD_TRY(cudaStreamBeginCaptureToGraph(ln.stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     const cudaError_t ce = capture_devloop_body(ln.d_loop, a, cond, ln.stream);
@@ -647,7 +647,7 @@ int devloop_lane_create(Server* sv, DevLoopHost& dl, DevLane& ln) {
     LUMRAD_TRY(ce);
     LUMRAD_TRY(ee);
     LUMRAD_TRY(cudaGraphInstantiate(&ln.exec, ln.graph, 0));
-    sv->fixed += (size_t)dl.max_tasks * kTaskRays * sizeof(RayResult) + sizeof(DevLoop);
+    sv->fixed += (size_t)dl.max_tasks * kTaskRays * kRayBytes + sizeof(DevLoop);
     return LUMRAD_OK;
 }
 
@@ -879,7 +879,7 @@ void devloop_destroy(Server* sv) {
         if (ln.graph) cudaGraphDestroy(ln.graph);
         cudaFree(ln.d_chunk_count);
         cudaFree(ln.d_chunk_off);
-        cudaFree(ln.d_ray_res);
+        cudaFree(ln.d_rays);
         cudaFree(ln.d_queue);
         cudaFree(ln.d_error);
         cudaFree(ln.d_loop);
@@ -910,7 +910,7 @@ void destroy_server(Server* sv) {
         if (sl.h_error) cudaFreeHost(sl.h_error);
         cudaFree(sl.d_queue);
         cudaFree(sl.d_error);
-        cudaFree(sl.d_ray_res);
+        cudaFree(sl.d_rays);
         if (sl.ev_done) cudaEventDestroy(sl.ev_done);
         if (sl.stream) cudaStreamDestroy(sl.stream);
     }
@@ -982,7 +982,7 @@ int lumrad_server_create(const LumRadServerSettings* s, LumRadServer* out) {
             *sl.h_error = 0;
             LUMRAD_TRY(cudaMemsetAsync(sl.d_queue, 0, kQueueWords * sizeof(unsigned long long), sl.stream));
             LUMRAD_TRY(cudaMemsetAsync(sl.d_error, 0, sizeof(int), sl.stream));
-            LUMRAD_TRY(cudaMalloc(&sl.d_ray_res, rays * sizeof(RayResult)));
+            LUMRAD_TRY(cudaMalloc(&sl.d_rays, rays * kRayBytes));
             // request packs sized up front so the serving loop rarely grows them
             const size_t pack = (size_t)16 << 20;
             LUMRAD_TRY(cudaMallocHost(&sl.h_pack, pack));
@@ -990,7 +990,7 @@ int lumrad_server_create(const LumRadServerSettings* s, LumRadServer* out) {
             LUMRAD_TRY(cudaMallocAsync(reinterpret_cast<void**>(&sl.d_pack), pack, sl.stream));
             sl.d_cap = pack;
             LUMRAD_TRY(cudaStreamSynchronize(sl.stream));
-            sv->fixed += rays * sizeof(RayResult) + pack + 2 * sizeof(unsigned long long) + sizeof(int);
+            sv->fixed += rays * kRayBytes + pack + 2 * sizeof(unsigned long long) + sizeof(int);
         }
         if (sv->fixed > sv->budget()) return fail(LUMRAD_ENOMEM, "the launch buffers alone exceed the HBM budget");
         return LUMRAD_OK;

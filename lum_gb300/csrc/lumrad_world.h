@@ -145,8 +145,7 @@ struct Context {
     int* d_error = nullptr;
     // rays of one march/finalize round (up to kChunkTasks * 32 rays), or of one march launch over
     // several passes (up to kMultiTasks * 32)
-    RayResult* d_ray_res = nullptr;
-    RayResult* d_ray_res2 = nullptr;           // the other ray buffer (consecutive passes alternate)
+    void* d_rays[2] = {nullptr, nullptr};      // kRayBytes * ray_cap each (consecutive passes alternate)
     int* d_ray_blk = nullptr;
     size_t ray_cap = 0;
     int ray_side = 0;
@@ -201,7 +200,7 @@ struct Context {
     unsigned long long* d_map_owner = nullptr;   // one word per voxel of the temporary palette slots
     size_t map_owner_cap = 0;
     // blockify staging, page-locked so the frame's uploads do not block the host: the working
-    // grid (W int16), compact grid (W uint16 at most), compact slots (n_slots + 128 ints) and
+    // grid (W int16), compact grid (uint16 at most), compact slots (n_slots + 128 ints) and
     // palette copies (n_slots int2); and the copies' device buffer
     uint8_t* h_blk = nullptr;
     int2* d_blk_copies = nullptr;

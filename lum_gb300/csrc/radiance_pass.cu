@@ -7,10 +7,12 @@
 //                    single tasks at the end; through a shared-memory block per CTA when the
 //                    launch has few tasks per warp).  A warp sets up a task's 32 rays in lock step
 //                    (hash seeds, direction, origin, 1/direction) into a 32-ray ring in shared
-//                    memory.  Its lanes march in a flat loop, two coarse steps per iteration; a
-//                    lane whose ray ends writes its RayResult (fraction, info, origin, direction)
-//                    and takes the next ray in ring order.  The ring is set up again as soon as its rays are handed out, so lanes
-//                    never wait for each other.
+//                    memory, takes their first coarse step there (38% of the demo's rays end on
+//                    it) and puts the rest into the ring.  Its lanes march in a flat loop, up to
+//                    three coarse steps per iteration; a lane whose ray ends writes its result
+//                    (fraction, info; the set-up wrote its origin and direction) and takes the next
+//                    ray in ring order.  The ring is set up again as soon as its rays are handed
+//                    out, so lanes never wait for each other.
 //   finalize_kernel  one warp per task, eight consecutive tasks per CTA, in lock step: the ray
 //                    read back, refine DDA, material, trilinear fetch of the previous radiance,
 //                    shading, xor-butterfly sum.  When R/32 divides 8 a probe's subgroups share a
@@ -28,7 +30,7 @@
 //
 // Exactness: see radiance_device.cuh.  Memory: both kernels test voxels through the compact
 // world (uint8 ids + occupancy bits, L1-resident; staged in shared memory by the march of a launch
-// over one world that fits); between the kernels each ray keeps its 32 B RayResult: 268 MB for a
+// over one world that fits); between the kernels each ray keeps 32 B (RayBuffer): 268 MB for a
 // single pass's round of 2^18 tasks, up to 537 MB for several passes, 1.07 GB for a batch's round
 // of 2^20.
 
@@ -41,31 +43,42 @@ namespace lumrad {
 namespace {
 
 // ---------------------------------------------------------------- march kernel
-// A ray is regular when each reciprocal of its direction is at most 2^100 in magnitude: no zero
-// component (only an exact cancellation in the set-up gives one, or one of a tiny magnitude).
-// Such a ray's march never meets a NaN or an infinity: its positions stay below 2^21 in
-// magnitude, its block corners within 32 of them, and its fraction grows by at least 0.5 - 2^-8
-// per step.  Hence, for it:
+// A ray is regular when each reciprocal of its direction is at most 2^100 in magnitude (no zero
+// component; only an exact cancellation in the set-up gives one, or one of a tiny magnitude) and
+// its probe lies in the world (its origin then does).  Such a ray's march never meets a NaN or an infinity: its positions
+// stay below 2^16 in magnitude, its block corners within 32 of them, and its fraction grows by at
+// least 0.5 - 2^-8 per step.  Hence, for it:
 //   (a) GLSL's min/max (y < x ? y : x) equal the hardware's min/max: they differ only on NaN and
 //       on the sign of a zero, and the skip's 0.01 floor maps both zeros alike;
-//   (b) a position lies outside [0, 16*size) exactly when it lies outside the grid lookup's
-//       range (-16, 16*size) or is negative (no position is -0: no origin is, and a sum is -0
-//       only if both terms are), so the exit test is the lookup's range test and the sign bits;
+//   (b) every position it looks up lies in (-1, 16*size + 1): a step adds 0.5 to the fraction, and
+//       the skip before it ends at the face of an air block it was in, up to the rounding of the
+//       axis with the largest direction component (at least 0.57: an error below 0.02) and the
+//       0.01 floor; a ray whose position is outside takes no further step.  So the lookup needs no
+//       range test (solid_inside);
 //   (c) the 2*max_dist+2 step bound is never reached: the fraction passes max_dist first;
-//   (d) the grid lookup can take the block index and the range test from trunc(p/16) in FP32
-//       (solid_at_tbp), which the empty-block skip needs anyway.
-// A warp whose rays are all regular marches with those forms (fewer compares and selects on the
-// integer/compare pipe, the one that limits this kernel); any other warp with the exact forms of
-// the general case.  Both give the same bits for a regular ray.
+//   (d) while the fraction before the skip is below `exit_fraction` no position is outside, so the
+//       exact test is made only for the lanes past it.
+// A warp whose rays are all regular marches with those forms; any other warp with the exact forms
+// of the general case.  Both give the same bits for a regular ray.
 __device__ __forceinline__ bool regular_ray(float ivx, float ivy, float ivz) {
     const float lim = 1.2676506002282294e30f;   // 2^100
     return fabsf(ivx) <= lim && fabsf(ivy) <= lim && fabsf(ivz) <= lim;
 }
 
+// A fraction below every one at which the position o + d*f of a regular ray is outside the world:
+// per axis the distance to the face ahead less 2^-7 (the position's roundings: below 2^-8 at 2^15)
+// over |d|, the least of them less 2^-20 of it (the quotient's roundings); at least 0.
+__device__ __forceinline__ float exit_fraction(float3 o, float3 d, float rx, float ry, float rz, float wx, float wy, float wz) {
+    const float ex = fmul(fsub(fabsf(fsub(d.x > 0.0f ? wx : 0.0f, o.x)), 0.0078125f), fabsf(rx));
+    const float ey = fmul(fsub(fabsf(fsub(d.y > 0.0f ? wy : 0.0f, o.y)), 0.0078125f), fabsf(ry));
+    const float ez = fmul(fsub(fabsf(fsub(d.z > 0.0f ? wz : 0.0f, o.z)), 0.0078125f), fabsf(rz));
+    return fmaxf(fmul(fminf(ex, fminf(ey, ez)), 0.99999905f), 0.0f);
+}
+
 // STAGE: one CTA of kStageWarps warps per SM, with the launch's compact world (compact grid and
 // occupancy masks, every world of the launch the same) copied into shared memory at the start;
 // lookups are then 32-bit-addressed shared loads (fewer address instructions, lower latency than
-// the L1-resident form: 8% off the demo step's march).  Used where the world fits beside the rays'
+// the L1-resident form: 8% off the demo step's march when it was introduced).  Used where the world fits beside the rays'
 // rings and parking space (98 KB of the 227 KB per CTA: a 64x64x16 world of 34 block types takes
 // 81 KB, and compact worlds up to ~125 KB fit); other launches (batches, servers, larger worlds,
 // hit records) read the world from global memory through L1.
@@ -78,15 +91,11 @@ static_assert(LUMRAD_MAX_CHUNK < (1 << 12) && kQueueCap <= LUMRAD_MAX_CHUNK, "a 
 constexpr int kWarpQueueDiv = 1;
 // launches with fewer tasks than this per warp claim through the CTA queue (march_kernel's CTAQ)
 constexpr int kCtaQueueTasksPerWarp = 32;
-// Rays a warp keeps set up in its shared-memory ring (a multiple of 32, a power of two): each slot
-// holds origin + ray index, direction, 1/direction + regular flag; a task (32 rays) is set up
-// whenever a ring's worth minus one task has been handed out.  One task: its 32 rays wait in the
-// ring while the lanes march the previous 32 (A/B on the demo step, bit-identical: 64-ray rings
-// 3.3% slower on a single pass and equal on 8 passes, 128-ray rings 11-12% slower: their shared
-// memory costs a CTA per SM).
-constexpr int kRingRays = kTaskRays;
-static_assert((kRingRays & (kRingRays - 1)) == 0 && kRingRays >= kTaskRays, "ring of whole tasks, a power of two");
-constexpr size_t kStageRingBytes = (size_t)kStageWarps * 3 * (kRingRays + kTaskRays) * sizeof(float4);
+// A warp's shared-memory ring holds the rays of one task (origin + ray index, direction + fraction,
+// 1/direction + exit fraction) that wait while the lanes march the previous ones; the next task is
+// set up once they are all handed out.  (Rings of two and four tasks: 3% and 11-12% slower on a
+// single pass, their shared memory costs a CTA per SM.)
+constexpr size_t kStageRingBytes = (size_t)kStageWarps * 6 * kTaskRays * sizeof(float4);
 
 // Tasks are claimed in two levels.  A CTA takes guided blocks from the launch's queue word
 // (remaining / (div * CTAs), clamped to [1, cap * warps per CTA]) into a shared-memory block word
@@ -156,6 +165,13 @@ __device__ __noinline__ long long refill_block(const LaunchArgs& la, int n_round
     return -1;
 }
 
+// What bounds it: instruction issue (84% of the slots on the demo's 8-pass launch, every world
+// lookup in shared memory).  Per 32-ray task that launch issues 912 warp instructions, of which the
+// set-up with its first step is about 350 and an iteration (3 steps of about 45 and the hand-out)
+// 200.  The launch: 436 -> 373 us, 452 -> 383 M warp instructions, with: lookups without range
+// tests or conversions for regular rays (solid_inside), x and y in register pairs, the first step
+// in the set-up, results and hand-outs once per three steps, and reciprocals and the square root
+// without their checks for operands that cannot occur.
 template <bool RECORD, bool STAGE = false, bool CTAQ = false>
 __global__ void __launch_bounds__(STAGE ? kStageWarps * 32 : kWarps * 32, STAGE ? 1 : 4)
 march_kernel(const __grid_constant__ LaunchArgs la) {
@@ -175,17 +191,17 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
             }
         }
     }
-    float4 (*s_ray)[3][kRingRays];    // set-up rays: origin, direction, (1/direction, regular)
+    float4 (*s_ray)[3][kTaskRays];    // the ring
     float4 (*s_park)[3][kTaskRays];   // in-flight ray state while the warp sets up
     const uint8_t* s_cg = nullptr;
     const uint16_t* s_rows = nullptr;
     if constexpr (STAGE) {
         extern __shared__ __align__(16) unsigned char s_dyn[];
-        s_ray = reinterpret_cast<float4 (*)[3][kRingRays]>(s_dyn);
-        s_park = reinterpret_cast<float4 (*)[3][kTaskRays]>(s_dyn + (size_t)kStageWarps * 3 * kRingRays * sizeof(float4));
+        s_ray = reinterpret_cast<float4 (*)[3][kTaskRays]>(s_dyn);
+        s_park = reinterpret_cast<float4 (*)[3][kTaskRays]>(s_dyn + (size_t)kStageWarps * 3 * kTaskRays * sizeof(float4));
         unsigned char* wb = s_dyn + kStageRingBytes;
         const WorldPass& w0 = la.worlds ? la.worlds[0] : la.single;
-        const int cg_bytes = w0.X * w0.Y * w0.Z * (w0.cgrid_wide ? 2 : 1);
+        const int cg_bytes = (w0.X + 1) * (w0.Y + 1) * (w0.Z + 1) * (w0.cgrid_wide ? 2 : 1);
         const int cg_pad = (cg_bytes + 15) & ~15;
         const int cb_bytes = w0.n_compact * 512;
         const uint8_t* gcg = reinterpret_cast<const uint8_t*>(w0.cgrid);
@@ -198,7 +214,7 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
         s_cg = wb;
         s_rows = reinterpret_cast<const uint16_t*>(wb + cg_pad);
     } else {
-        __shared__ float4 a_ray[kWarps][3][kRingRays];
+        __shared__ float4 a_ray[kWarps][3][kTaskRays];
         __shared__ float4 a_park[kWarps][3][kTaskRays];
         s_ray = a_ray;
         s_park = a_park;
@@ -229,26 +245,24 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
     const WorldPass* wp = &la.single;
     MarchView mv{0, 0, 0, 0, nullptr, nullptr};
     float wx = 0.0f, wy = 0.0f, wz = 0.0f, max_dist = 0.0f;
+    unsigned kb = 0;
     int max_steps = 0;
     int w_begin = 0, w_end = 0;
-    // FIFO ring: ray q of the issue order lives in ring slot q mod kRingRays; `loaded` rays have
-    // been set up, `issued` handed out
+    // the ring: rays [issued, loaded) of the last task set up wait to be handed out; ring_fast: all
+    // of them are regular
     int issued = 0, loaded = 0;
+    bool ring_fast = true;
     int tb = 0, te = 0;          // grabbed task chunk [tb, te)
     bool exhausted = false;
     int pending = -1;            // grabbed task of another world, waiting for the lanes to drain
 
     // lane ray state
     int my = -1;                 // round-relative index of the lane's ray, -1 if idle
-    float ox = 0, oy = 0, oz = 0, dx = 0, dy = 0, dz = 0, ivx = 0, ivy = 0, ivz = 0, cx = 0, cy = 0, cz = 0, frac = 0;
+    f32x2 oxy = 0, dxy = 0, ivxy = 0, cxy = 0;   // x and y of origin, direction, 1/direction, corner
+    float oz = 0, dz = 0, ivz = 0, cz = 0, frac = 0;
     int steps = 0;
-    bool reg = true;             // the lane's ray is regular (see regular_ray)
+    float fexit = 0.0f;          // exit_fraction over the axes; -1: the ray is not regular
 
-    // Tasks are claimed in two levels.  A CTA takes guided blocks from the launch's queue word
-    // (remaining / (div * CTAs), clamped to [1, cap * warps per CTA]) into a shared-memory block;
-    // its warps take single tasks from that block with a shared-memory atomic, and the warp that
-    // finds it empty fetches the next block under a shared lock.  The global word sees one claim
-    // per CTA block instead of one per warp chunk, and warps balance at single tasks.
     // Claims: CTAQ, through the CTA's block (claim_from_block, refill_block; launches with few tasks
     // per warp, such as a single pass: the warps balance at single tasks); else straight from the
     // launch's queue word in guided chunks of remaining / (div * warps), clamped to [1, cap]
@@ -284,122 +298,141 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
         }
         return tb;
     };
-    auto corner = [&]() {
-        cx = dx > 0.0f ? 16.0f : 0.0f;
-        cy = dy > 0.0f ? 16.0f : 0.0f;
-        cz = dz > 0.0f ? 16.0f : 0.0f;
+    auto corner = [&](float dx, float dy) {   // the far corner's offset in a block, less kBlockBias (exact)
+        cxy = pack2(dx > 0.0f ? 16.0f - kBlockBias : -kBlockBias, dy > 0.0f ? 16.0f - kBlockBias : -kBlockBias);
+        cz = dz > 0.0f ? 16.0f - kBlockBias : -kBlockBias;
     };
     // hand the next rays in ring order to the lanes in `need`
     auto assign = [&](unsigned need) {
-        const int avail = loaded - issued;
-        const int rank = __popc(need & lt_mask);
-        if (((need >> lane) & 1u) && rank < avail) {
-            const int q = issued + rank;
-            const int slot = q & (kRingRays - 1);
+        const int slot = issued + __popc(need & lt_mask);
+        if (((need >> lane) & 1u) && slot < loaded) {
             const float4 o4 = so[slot], d4 = sd[slot], i4 = si[slot];
             my = __float_as_int(o4.w);   // the ray's round-relative index, stored with its origin
-            ox = o4.x; oy = o4.y; oz = o4.z;
-            dx = d4.x; dy = d4.y; dz = d4.z;
-            ivx = i4.x; ivy = i4.y; ivz = i4.z;
-            reg = i4.w != 0.0f;
-            corner();
-            frac = 0.0f;
-            steps = 0;
+            oxy = pack2(o4.x, o4.y); oz = o4.z;
+            dxy = pack2(d4.x, d4.y); dz = d4.z;
+            ivxy = pack2(i4.x, i4.y); ivz = i4.z;
+            fexit = i4.w;
+            corner(d4.x, d4.y);
+            frac = d4.w;
+            steps = d4.w != 0.0f ? 1 : 0;   // a first step in the set-up leaves at least 0.5
         }
-        issued += min(avail, __popc(need));
+        issued = min(loaded, issued + __popc(need));
     };
+    // ray i has ended, its last lookup at p
+    auto end_ray = [&](int i, float px, float py, float pz, bool solid, uint32_t info) {
+        if (RECORD) {
+            int blk;
+            const int v = voxel_value(*wp, f2i(px), f2i(py), f2i(pz), blk);
+            if (solid) info |= (uint32_t)v << 16;
+            la.ray_blk[i] = blk;
+        }
+        __stcg(la.rays.res + i, make_uint2(__float_as_uint(frac), info));
+    };
+    // One coarse step (CastRay_fast, radiance.comp:198-244) of the lane's regular ray, straight-line
+    // (the empty-block skip, radiance.comp:215-226, is formed for every lane and selected where the
+    // block is air); true if the ray may have ended: `solid`, or at p or frac (ray_ended).
+    float f1 = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f;
+    bool solid = false;
+    auto step = [&](bool wide) -> bool {
+        f1 = fadd(frac, 0.5f);
+        const f32x2 pxy = add_product2(oxy, mul2(dxy, pack2(f1, f1)));
+        unpack2(pxy, px, py);
+        pz = fadd(oz, fmul(dz, f1));
+        const float qx = fabsf(px), qy = fabsf(py), qz = fabsf(pz);
+        const float bx = __fadd_rz(qx, kBlockBias), by = __fadd_rz(qy, kBlockBias), bz = __fadd_rz(qz, kBlockBias);
+        const int cid = cell_id<STAGE>(STAGE ? s_cg : mv.cgrid, cell_inside(mv.X + 1, mv.Y + 1, kb, bx, by, bz), wide);
+        solid = solid_inside<STAGE>(STAGE ? s_rows : reinterpret_cast<const uint16_t*>(mv.cbits), cid, qx, qy, qz);
+        float tx, ty;
+        // to the face ahead (b + c is exact)
+        unpack2(sub_product2(mul2(add2(pack2(bx, by), cxy), ivxy), mul2(pxy, ivxy)), tx, ty);
+        const float tz = fsub(fmul(fadd(bz, cz), ivz), fmul(pz, ivz));
+        const float sk = fmaxf(fminf(tx, fminf(ty, tz)), 0.01f);
+        frac = cid == 0 ? fadd(f1, sk) : f1;
+        steps++;
+        return solid || f1 >= fexit || frac >= max_dist;
+    };
+    auto ray_ended = [&]() -> bool {
+        return solid || frac >= max_dist || px < 0.0f || py < 0.0f || pz < 0.0f || px >= wx || py >= wy || pz >= wz;
+    };
+    auto hit_info = [&]() -> uint32_t { return (uint32_t)steps | (solid ? 1u << 24 : 0u); };
     auto more_tasks = [&]() { return pending < 0 && !(exhausted && tb >= te); };
 
-    // The coarse march (CastRay_fast, radiance.comp:198-244) of the lanes' rays, two coarse steps
-    // per iteration (a lane whose ray ends in the first takes no second: the warp's vote and
-    // hand-out run once per two steps), until the ring has room for a task while tasks may remain,
-    // or no lane has a ray; a FAST loop also ends when a lane takes a ray that is not regular.
+    // The coarse march of the lanes' rays, up to three steps per iteration (two: 1-2% slower, four:
+    // equal): a lane whose ray ends takes no further one, and the ended rays' results are written
+    // and their lanes given new rays once per iteration.  Runs until the ring is empty while tasks
+    // may remain, or no lane has a ray.  FAST: every lane's ray and the ring's are regular.
     auto march = [&](auto fast_tag, auto wide_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
         constexpr bool WIDE = decltype(wide_tag)::value;
-        const uint8_t* cgp = STAGE ? s_cg : mv.cgrid;
-        const uint16_t* rowp = STAGE ? s_rows : reinterpret_cast<const uint16_t*>(mv.cbits);
         while (true) {
             bool fin = false;
-#pragma unroll
-            for (int u = 0; u < 2; u++) {   // (3 or 4 steps per iteration measured 0.2-0.7% slower)
-                // Straight-line: every lane runs the step (an idle lane's stale ray reads only
-                // in-range cells and its results are dropped) and the empty-block skip
-                // (radiance.comp:215-226) is formed for every lane and selected where the block is
-                // air: no divergent branch per step (3% fewer instructions than branching).  The
-                // block's low corner (ix/16)*16 with ix = trunc(px) is trunc(px/16)*16, formed in
-                // FP32 (exact: px/16 and the product by 16 are exact, |px| < 2^21; a NaN px gives
-                // a NaN skip either way).
-                const bool act = my >= 0;
-                const float f1 = fadd(frac, 0.5f);
-                const int st = steps + 1;
-                const float px = fadd(ox, fmul(dx, f1));
-                const float py = fadd(oy, fmul(dy, f1));
-                const float pz = fadd(oz, fmul(dz, f1));
-                const int ix = f2i(px), iy = f2i(py), iz = f2i(pz);
-                const float tbx = truncf(fmul(px, 0.0625f)), tby = truncf(fmul(py, 0.0625f)), tbz = truncf(fmul(pz, 0.0625f));
-                int cid;
-                bool in_range = true;
-                const bool solid =
-                    FAST ? solid_at_tbp<WIDE, STAGE>(cgp, rowp, mv.X, mv.Y, mv.Z, tbx, tby, tbz, ix, iy, iz, cid, in_range)
-                         : solid_at_p<WIDE, STAGE>(cgp, rowp, mv.X, mv.Y, mv.Z, ix, iy, iz, cid);
-                // tb*16 is exact (tb = trunc(p/16), an integer of at most |p|/16)
-                const float bx = fadd_exact_mul(cx, tbx, 16.0f);
-                const float by = fadd_exact_mul(cy, tby, 16.0f);
-                const float bz = fadd_exact_mul(cz, tbz, 16.0f);
-                const float tx = fadd(fmul(bx, ivx), fmul(-px, ivx));
-                const float ty = fadd(fmul(by, ivy), fmul(-py, ivy));
-                const float tz = fadd(fmul(bz, ivz), fmul(-pz, ivz));
-                const float sk = FAST ? fmaxf(fminf(tx, fminf(ty, tz)), 0.01f) : gmax(gmin(tx, gmin(ty, tz)), 0.01f);
-                const float f2 = cid == 0 ? fadd(f1, sk) : f1;
-                bool out;
-                // a regular ray's position is outside [0, 16*size) on an axis exactly when it is
-                // outside the lookup's range (-16, 16*size) or negative (no position is -0): one
-                // test of the three sign bits beside the lookup's own range test
-                if (FAST)
-                    out = !in_range || (int)(__float_as_uint(px) | __float_as_uint(py) | __float_as_uint(pz)) < 0 ||
-                          f2 >= max_dist;
-                else
-                    out = px < 0.0f || py < 0.0f || pz < 0.0f || px >= wx || py >= wy || pz >= wz || f2 >= max_dist;
-                const bool capped = !FAST && st >= max_steps;
-                frac = f2;
-                steps = st;
-                const bool f = act && (solid || out || capped);
-                if (f) {
-                    uint32_t info = (uint32_t)st | (solid ? (1u << 24) : (out ? 0u : (1u << 25)));
-                    if (RECORD) {
-                        int blk;
-                        const int v = voxel_value(*wp, ix, iy, iz, blk);
-                        if (solid) info |= (uint32_t)v << 16;
-                        la.ray_blk[my] = blk;
+            if constexpr (FAST) {
+                if (my >= 0) {
+                    fin = step(WIDE);
+                    if (!fin) fin = step(WIDE);
+                    if (!fin) fin = step(WIDE);
+                }
+                if (fin) {
+                    fin = ray_ended();
+                    if (fin) {
+                        end_ray(my, px, py, pz, solid, hit_info());
+                        my = -1;
                     }
-                    uint4* rr = reinterpret_cast<uint4*>(la.ray_res + my);   // RayResult
-                    __stcg(rr, make_uint4(__float_as_uint(f2), info, __float_as_uint(ox), __float_as_uint(oy)));
-                    __stcg(rr + 1, make_uint4(__float_as_uint(oz), __float_as_uint(dx), __float_as_uint(dy),
-                                              __float_as_uint(dz)));
-                    my = -1;
-                    fin = true;
+                }
+            } else {
+                // the general form: GLSL's min and max, the step bound, range-tested lookups
+                const uint8_t* cgp = STAGE ? s_cg : mv.cgrid;
+                const uint16_t* rowp = STAGE ? s_rows : reinterpret_cast<const uint16_t*>(mv.cbits);
+                float ox, oy, dx, dy, ivx, ivy, cx, cy;
+                unpack2(oxy, ox, oy);
+                unpack2(dxy, dx, dy);
+                unpack2(ivxy, ivx, ivy);
+                unpack2(cxy, cx, cy);
+                for (int u = 0; u < 2 && my >= 0; u++) {
+                    const float f = fadd(frac, 0.5f);
+                    const float x = fadd(ox, fmul(dx, f)), y = fadd(oy, fmul(dy, f)), z = fadd(oz, fmul(dz, f));
+                    int cid;
+                    const bool hit = solid_at_p<WIDE, STAGE>(cgp, rowp, mv.X, mv.Y, mv.Z, f2i(x), f2i(y), f2i(z), cid);
+                    // the block's low corner (ix/16)*16 with ix = trunc(x) is trunc(x/16)*16, exact
+                    // in FP32 (a NaN x gives a NaN skip either way)
+                    const float bx = fadd_exact_mul(fadd(cx, kBlockBias), truncf(fmul(x, 0.0625f)), 16.0f);
+                    const float by = fadd_exact_mul(fadd(cy, kBlockBias), truncf(fmul(y, 0.0625f)), 16.0f);
+                    const float bz = fadd_exact_mul(fadd(cz, kBlockBias), truncf(fmul(z, 0.0625f)), 16.0f);
+                    const float tx = fadd(fmul(bx, ivx), fmul(-x, ivx));
+                    const float ty = fadd(fmul(by, ivy), fmul(-y, ivy));
+                    const float tz = fadd(fmul(bz, ivz), fmul(-z, ivz));
+                    const float sk = gmax(gmin(tx, gmin(ty, tz)), 0.01f);
+                    frac = cid == 0 ? fadd(f, sk) : f;
+                    steps++;
+                    const bool out = x < 0.0f || y < 0.0f || z < 0.0f || x >= wx || y >= wy || z >= wz || frac >= max_dist;
+                    if (hit || out || steps >= max_steps) {
+                        end_ray(my, x, y, z, hit, (uint32_t)steps | (hit ? (1u << 24) : (out ? 0u : (1u << 25))));
+                        my = -1;
+                        fin = true;
+                    }
                 }
             }
             const unsigned fm = __ballot_sync(kFull, fin);
             if (fm) {
                 assign(fm);
-                if (!__any_sync(kFull, my >= 0) || (loaded - issued <= kRingRays - kTaskRays && more_tasks())) break;
-                if (FAST && !__all_sync(kFull, reg || my < 0)) break;
+                if (loaded == issued && (more_tasks() || !__any_sync(kFull, my >= 0))) break;
             }
         }
     };
 
     while (true) {
-        // 1. set up tasks into the ring's free room (32 slots free once their rays are handed out)
-        const bool refill = loaded - issued <= kRingRays - kTaskRays && (pending >= 0 || more_tasks());
-        if (refill && my >= 0) {   // park: the setup needs the registers
-            s_park[wib][0][lane] = make_float4(ox, oy, oz, frac);
-            s_park[wib][1][lane] = make_float4(dx, dy, dz, __int_as_float(steps));
-            s_park[wib][2][lane] = make_float4(ivx, ivy, ivz, reg ? 1.0f : 0.0f);
+        // 1. set up tasks until one leaves rays in the ring
+        const bool refill = loaded == issued && (pending >= 0 || more_tasks());
+        if (refill && my >= 0) {   // park: the set-up needs the registers
+            float x, y;
+            unpack2(oxy, x, y);
+            s_park[wib][0][lane] = make_float4(x, y, oz, frac);
+            unpack2(dxy, x, y);
+            s_park[wib][1][lane] = make_float4(x, y, dz, __int_as_float(steps));
+            unpack2(ivxy, x, y);
+            s_park[wib][2][lane] = make_float4(x, y, ivz, fexit);
         }
-        bool loaded_now = false;
-        while (refill && loaded - issued <= kRingRays - kTaskRays) {
+        while (refill && loaded == issued) {
             const int t = next_task();
             if (t < 0) break;
             if (t < w_begin || t >= w_end) {
@@ -412,13 +445,14 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
                 // compact world with the same bound (passes of one context), whose rays march alike
                 const bool alike = reinterpret_cast<const uint8_t*>(wq->cgrid) == mv.cgrid &&
                                    wq->max_dist == max_dist;
-                if (!alike && (__any_sync(kFull, my >= 0) || loaded > issued)) {
+                if (!alike && __any_sync(kFull, my >= 0)) {
                     if (pending != t) tb++;
                     pending = t;
                     break;
                 }
                 wp = wq;
                 mv = march_view(*wp);
+                kb = cell_bias(mv.X + 1, mv.Y + 1);
                 wx = fmul((float)mv.X, 16.0f); wy = fmul((float)mv.Y, 16.0f); wz = fmul((float)mv.Z, 16.0f);
                 max_dist = wp->max_dist;
                 max_steps = wp->max_steps;
@@ -431,35 +465,59 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
             const int nsub = wp->R >> 5;
             const int g = div_nsub(t_local, nsub);
             float3 o, d;
-            setup_ray(*wp, g, (t_local - g * nsub) * kTaskRays + lane, o, d);
-            const int slot = (loaded & (kRingRays - 1)) + lane;
-            const float4 o4 = make_float4(o.x, o.y, o.z, __int_as_float((t - la.chunk_begin) * kTaskRays + lane));
-            const float4 d4 = make_float4(d.x, d.y, d.z, 0.0f);
-            so[slot] = o4;
-            sd[slot] = d4;
-            const float rx = __frcp_rn(d.x), ry = __frcp_rn(d.y), rz = __frcp_rn(d.z);
-            si[slot] = make_float4(rx, ry, rz, regular_ray(rx, ry, rz) ? 1.0f : 0.0f);
-            loaded += kTaskRays;
-            loaded_now = true;
+            const bool inside = setup_ray(*wp, g, (t_local - g * nsub) * kTaskRays + lane, o, d);
+            const int idx = (t - la.chunk_begin) * kTaskRays + lane;
+            __stcg(la.rays.od + idx, make_float4(o.x, o.y, o.z, d.x));
+            __stcg(la.rays.dd + idx, make_float2(d.y, d.z));
+            float rx = rcp_normal(d.x), ry = rcp_normal(d.y), rz = rcp_normal(d.z);
+            const bool regular = inside && regular_ray(rx, ry, rz);
+            if (!regular) {
+                rx = __frcp_rn(d.x);
+                ry = __frcp_rn(d.y);
+                rz = __frcp_rn(d.z);
+            }
+            // the rays' first step here, where all 32 lanes take it; the rays that go on into the ring
+            oxy = pack2(o.x, o.y); oz = o.z;
+            dxy = pack2(d.x, d.y); dz = d.z;
+            ivxy = pack2(rx, ry); ivz = rz;
+            fexit = regular ? exit_fraction(o, d, rx, ry, rz, wx, wy, wz) : -1.0f;
+            corner(d.x, d.y);
+            frac = 0.0f;
+            steps = 0;
+            bool on = true;
+            ring_fast = __all_sync(kFull, regular);
+            if (ring_fast && step(mv.wide) && ray_ended()) {
+                end_ray(idx, px, py, pz, solid, hit_info());
+                on = false;
+            }
+            const unsigned sm = __ballot_sync(kFull, on);
+            if (on) {
+                const int slot = __popc(sm & lt_mask);
+                so[slot] = make_float4(o.x, o.y, o.z, __int_as_float(idx));
+                sd[slot] = make_float4(d.x, d.y, d.z, frac);
+                si[slot] = make_float4(rx, ry, rz, fexit);
+            }
+            issued = 0;
+            loaded = __popc(sm);
         }
         __syncwarp();
         if (refill && my >= 0) {
             const float4 a = s_park[wib][0][lane], b = s_park[wib][1][lane], c = s_park[wib][2][lane];
-            ox = a.x; oy = a.y; oz = a.z; frac = a.w;
-            dx = b.x; dy = b.y; dz = b.z; steps = __float_as_int(b.w);
-            ivx = c.x; ivy = c.y; ivz = c.z; reg = c.w != 0.0f;
-            corner();
+            oxy = pack2(a.x, a.y); oz = a.z; frac = a.w;
+            dxy = pack2(b.x, b.y); dz = b.z; steps = __float_as_int(b.w);
+            ivxy = pack2(c.x, c.y); ivz = c.z; fexit = c.w;
+            corner(b.x, b.y);
         }
         // 2. idle lanes take rays
         assign(__ballot_sync(kFull, my < 0));
         if (!__any_sync(kFull, my >= 0)) {
             // nothing in flight and nothing set up: no task was left (a task of another world
             // would have been set up above, the lanes being drained)
-            if ((pending >= 0 || loaded_now) && lane == 0) atomicOr(la.error, 1);
+            if ((pending >= 0 || loaded > issued) && lane == 0) atomicOr(la.error, 1);
             break;
         }
         // 3. march
-        const bool fast = __all_sync(kFull, reg || my < 0);
+        const bool fast = ring_fast && __all_sync(kFull, fexit >= 0.0f || my < 0);
         if (mv.wide) {
             if (fast) march(std::true_type{}, std::true_type{});
             else march(std::false_type{}, std::true_type{});
@@ -539,13 +597,13 @@ __device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, 
     const bool local = nsub > 1 && (kFinWarps % nsub) == 0 && (wp->task_begin % kFinWarps) == 0;
     float3 v = make_float3(0.0f, 0.0f, 0.0f);
     if (valid) {
-        const long long idx = (long long)(t - la.ray_origin) * kTaskRays + lane;
-        const uint4* rr = reinterpret_cast<const uint4*>(la.ray_res + idx);   // RayResult
-        const uint4 r0 = __ldcg(rr), r1 = __ldcg(rr + 1);
-        const uint2 res = make_uint2(r0.x, r0.y);
+        const int idx = (t - la.ray_origin) * kTaskRays + lane;
+        const uint2 res = __ldcg(la.rays.res + idx);
+        const float4 od = __ldcg(la.rays.od + idx);
+        const float2 dd = __ldcg(la.rays.dd + idx);
         const int blk = RECORD ? __ldcg(la.ray_blk + idx) : 0;
-        const float3 o = make_float3(__uint_as_float(r0.z), __uint_as_float(r0.w), __uint_as_float(r1.x));
-        const float3 d = make_float3(__uint_as_float(r1.y), __uint_as_float(r1.z), __uint_as_float(r1.w));
+        const float3 o = make_float3(od.x, od.y, od.z);
+        const float3 d = make_float3(od.w, dd.x, dd.y);
         uint32_t lookups;
         float3 L, u;
         float4 m;
@@ -684,7 +742,7 @@ size_t stage_bytes(const WorldPass& w) {
         ready[dev] = true;
     }
     if (w.n_compact <= 0) return 0;
-    const size_t cg = ((size_t)w.X * w.Y * w.Z * (w.cgrid_wide ? 2 : 1) + 15) & ~(size_t)15;
+    const size_t cg = (compact_cells(w.X, w.Y, w.Z) * (w.cgrid_wide ? 2 : 1) + 15) & ~(size_t)15;
     const size_t bytes = kStageRingBytes + cg + (size_t)w.n_compact * 512;
     return bytes <= (size_t)max_optin[dev] ? bytes : 0;
 }
@@ -913,8 +971,10 @@ __global__ void apply_edits_kernel(const WorldPass* __restrict__ worlds, const E
     const EditRecord e = edits[i];
     const WorldPass& w = worlds[e.world];
     const_cast<int16_t*>(w.grid)[e.index] = (int16_t)e.block;
-    if (w.cgrid_wide) static_cast<uint16_t*>(const_cast<void*>(w.cgrid))[e.index] = (uint16_t)e.compact;
-    else static_cast<uint8_t*>(const_cast<void*>(w.cgrid))[e.index] = (uint8_t)e.compact;
+    const int x = e.index % w.X, q = e.index / w.X;
+    const size_t cell = x + (size_t)(w.X + 1) * (q % w.Y + (size_t)(w.Y + 1) * (q / w.Y));
+    if (w.cgrid_wide) static_cast<uint16_t*>(const_cast<void*>(w.cgrid))[cell] = (uint16_t)e.compact;
+    else static_cast<uint8_t*>(const_cast<void*>(w.cgrid))[cell] = (uint8_t)e.compact;
 }
 
 }  // namespace
@@ -949,14 +1009,17 @@ namespace lumrad {
 namespace {
 
 constexpr int kNoAllocMaxBlocks = LUMRAD_NOALLOC_MAX_BLOCKS;
-constexpr int kNoAllocRoundTasks = 4096;
+constexpr int kNoAllocRoundTasks = 3840;
+// the most cells of a compact grid of kNoAllocMaxBlocks blocks (compact_cells): a world of one
+// block's height, 2047 blocks long
+constexpr size_t kNoAllocMaxCells = 2 * ((size_t)kNoAllocMaxBlocks + 2047 + kNoAllocMaxBlocks / 2047 + 1);
 constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 // byte offsets of the parts of the array
-constexpr size_t kNaCgrid = 0;                                                        // uint16 per block
-constexpr size_t kNaCbits = align256(kNaCgrid + 2 * (size_t)kNoAllocMaxBlocks);      // 512 B per compact id
-constexpr size_t kNaRayRes = align256(kNaCbits + (size_t)(LUMRAD_MAX_BLOCK_SLOTS + 2) * 512);
+constexpr size_t kNaCgrid = 0;                                                        // uint16 per cell
+constexpr size_t kNaCbits = align256(kNaCgrid + 2 * kNoAllocMaxCells);                 // 512 B per compact id
+constexpr size_t kNaRays = align256(kNaCbits + (size_t)(LUMRAD_MAX_BLOCK_SLOTS + 2) * 512);
 // the direction tables for R = 32, 64, 128, 256 back to back (480 entries), uploaded once per device
-constexpr size_t kNaDirs = align256(kNaRayRes + (size_t)kNoAllocRoundTasks * kTaskRays * sizeof(RayResult));
+constexpr size_t kNaDirs = align256(kNaRays + (size_t)kNoAllocRoundTasks * kTaskRays * kRayBytes);
 constexpr int kNaDirEntries = 32 + 64 + 128 + 256;
 constexpr size_t kNaQueue = align256(kNaDirs + kNaDirEntries * sizeof(float4));
 constexpr size_t kNaError = kNaQueue + kQueueWords * sizeof(unsigned long long);
@@ -977,9 +1040,12 @@ namespace {
 
 // Compact ids for the no-allocation form: 0 for block id 0 (palette slot 0), 1 + slot for a
 // non-zero id with a palette slot, n_slots + 1 (all empty) for any other id.
-__global__ void noalloc_compact_grid(const int16_t* __restrict__ grid, int W, int n_slots, uint16_t* __restrict__ cgrid) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < W; i += gridDim.x * blockDim.x) {
-        const int b = grid[i];
+__global__ void noalloc_compact_grid(const int16_t* __restrict__ grid, int X, int Y, int Z, int n_slots,
+                                     uint16_t* __restrict__ cgrid) {
+    const int n = (X + 1) * (Y + 1) * (Z + 1);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int x = i % (X + 1), q = i / (X + 1), y = q % (Y + 1), z = q / (Y + 1);
+        const int b = x < X && y < Y && z < Z ? grid[x + X * (y + Y * z)] : 0;
         const int slot = b < 0 ? b + 64 : b;
         const bool has = b >= -63 && slot < n_slots;
         cgrid[i] = (uint16_t)(b == 0 ? 0 : (has ? slot + 1 : n_slots + 1));
@@ -1091,7 +1157,7 @@ extern "C" int lumrad_radiance_pass_noalloc(const int* world_size, const int16_t
     // reads it), and this call's inputs derived into the array
     LUMRAD_TRY(cudaMemsetAsync(queue, 0, kQueueWords * sizeof(unsigned long long), stream));
     LUMRAD_TRY(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), stream));
-    noalloc_compact_grid<<<256, 256, 0, stream>>>(d_grid, (int)W, n_slots, cgrid);
+    noalloc_compact_grid<<<256, 256, 0, stream>>>(d_grid, world_size[0], world_size[1], world_size[2], n_slots, cgrid);
     noalloc_compact_bits<<<256, 256, 0, stream>>>(d_palette, n_slots, cbits);
     LUMRAD_TRY(cudaGetLastError());
     // probes outside the list keep their value
@@ -1134,7 +1200,7 @@ extern "C" int lumrad_radiance_pass_noalloc(const int* world_size, const int16_t
     la.n_tasks = n_tasks;
     la.queue = queue;
     la.error = error;
-    la.ray_res = reinterpret_cast<RayResult*>(base + kNaRayRes);
+    la.rays = ray_buffer(base + kNaRays, (size_t)kNoAllocRoundTasks * kTaskRays);
     const int blocks = march_grid(false, nd->num_sms, std::min<long long>(n_tasks, kNoAllocRoundTasks));
     la.total_warps = blocks * kWarps;
     for (long long c0 = 0; c0 < n_tasks; c0 += kNoAllocRoundTasks) {

@@ -195,7 +195,8 @@ __global__ void apply_kernel(DevLoop* L) {
         const int b = ed.block;
         const int c = (b >= -64 && b < w.n_cmap - 64) ? (int)w.cmap[b + 64] : w.empty_c;
         const_cast<int16_t*>(w.pass.grid)[idx] = (int16_t)b;
-        static_cast<uint8_t*>(const_cast<void*>(w.pass.cgrid))[idx] = (uint8_t)c;
+        const size_t cell = ed.x + (size_t)(w.pass.X + 1) * (ed.y + (size_t)(w.pass.Y + 1) * ed.z);
+        static_cast<uint8_t*>(const_cast<void*>(w.pass.cgrid))[cell] = (uint8_t)c;
     }
 }
 
