@@ -44,8 +44,8 @@ extern "C" long long arith_check(int which) {
     unsigned long long h = 0;
     if (cudaMalloc(&d, 8) != cudaSuccess || cudaMemset(d, 0, 8) != cudaSuccess) return -1;
     const int blocks = (1 << 23) / 256;
-    if (which == 0) rcp_check<<<blocks, 256>>>(d, -100, 3);
-    if (which == 1) sqrt_check<<<blocks, 256>>>(d, -4, 4);
+    if (which == 0) rcp_check<<<blocks, 256>>>(d, -100, 20);
+    if (which == 1) sqrt_check<<<blocks, 256>>>(d, -40, 40);
     if (which == 2) pair_check<<<blocks, 256>>>(d, 1u);
     if (which == 3) pair_sub_check<<<blocks, 256>>>(d, 2u);
     const cudaError_t e = cudaMemcpy(&h, d, 8, cudaMemcpyDeviceToHost);
