@@ -343,9 +343,9 @@ int DeviceWorld::fill_pass(const short4* d_req, int n, const LumRadPassParams& p
     w.alpha = p.blend;
     w.one_minus_alpha = 1.0f - p.blend;
     w.seed = (uint32_t)p.time_seed;
-    w.inv_dim[0] = exact_inverse(X);
-    w.inv_dim[1] = exact_inverse(Y);
-    w.inv_dim[2] = exact_inverse(Z);
+    w.inv_dim[0] = 1.0f / (float)X;
+    w.inv_dim[1] = 1.0f / (float)Y;
+    w.inv_dim[2] = 1.0f / (float)Z;
     w.inv_nsub = exact_inverse(R / 32);
     w.dirs = dirs;
     w.hits = p.record_hits ? d_hits : nullptr;

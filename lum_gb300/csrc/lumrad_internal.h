@@ -34,7 +34,7 @@ constexpr int kMultiTasks = 1 << 19;
 // buffer (RayBuffer): origin and direction x (16 B), direction y and z (8 B), both written by the
 // set-up, one task's 32 rays side by side; and the result (8 B): the coarse fraction's bits and
 // the info word (bits 0-15 coarse steps, 16-23 coarse voxel (records only), 24 hit, 25 stopped by
-// the step bound), written when the ray ends.  The finalize reads the ray back instead of setting
+// the step bound, 26 regular), written when the ray ends.  The finalize reads the ray back instead of setting
 // it up again.  (Rays end a few lanes at a time: one 32-byte record per ending ray took the march's
 // loop two 16-byte stores and their register moves per iteration where the set-up's whole-warp
 // stores are two per task.)
@@ -83,7 +83,7 @@ struct WorldPass {
     int max_steps;               // 2*max_dist + 2
     float alpha, one_minus_alpha;
     uint32_t seed;               // time seed
-    float inv_dim[3];            // 1/X, 1/Y, 1/Z where that is exact (power of two), else 0
+    float inv_dim[3];            // 1/X, 1/Y, 1/Z rounded to nearest
     float inv_nsub;              // 1/(R/32) where exact, else 0
     const float4* dirs;          // R spherical-Fibonacci directions
     LumRadHit* hits;             // per-ray records, or nullptr

@@ -13,13 +13,13 @@
 //                    (fraction, info; the set-up wrote its origin and direction) and takes the next
 //                    ray in ring order.  The ring is set up again as soon as its rays are handed
 //                    out, so lanes never wait for each other.
-//   finalize_kernel  one warp per task, eight consecutive tasks per CTA, in lock step: the ray
-//                    read back, refine DDA, material, trilinear fetch of the previous radiance,
-//                    shading, xor-butterfly sum.  When R/32 divides 8 a probe's subgroups share a
-//                    CTA and their means are summed in order from shared memory (a lean
-//                    instantiation, 8 CTAs per SM, 6 in the device loop's persistent form, when every
-//                    probe of the launch does); otherwise through global scratch and a per-probe
-//                    counter.  Lookup and hit counters are summed per CTA.
+//   finalize_kernel  eight consecutive tasks per CTA of two warps: the rays read back, the hits
+//                    packed 32 to a warp for the refine DDA, material, trilinear fetch of the
+//                    previous radiance and shading; then one lane per task and channel for the
+//                    xor-butterfly sum.  When R/32 divides 8 a probe's subgroups share a CTA and
+//                    their means are summed in order (a lean instantiation when every probe of the
+//                    launch does); otherwise through global scratch and a per-probe counter.
+//                    Lookup and hit counters are summed per CTA.
 //
 // Several passes of one context (launch_passes): one march launch over all their tasks (the
 // traversal does not read the radiance volume), then each pass's finalize in order, each launched
@@ -354,7 +354,8 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
     auto ray_ended = [&]() -> bool {
         return solid || frac >= max_dist || px < 0.0f || py < 0.0f || pz < 0.0f || px >= wx || py >= wy || pz >= wz;
     };
-    auto hit_info = [&]() -> uint32_t { return (uint32_t)steps | (solid ? 1u << 24 : 0u); };
+    // (a hit in a block of id 0 has the skip in its fraction, and the refine starts past it: general)
+    auto hit_info = [&]() -> uint32_t { return (uint32_t)steps | (frac == f1 ? kInfoRegular : 0u) | (solid ? kInfoHit : 0u); };
     auto more_tasks = [&]() { return pending < 0 && !(exhausted && tb >= te); };
 
     // The coarse march of the lanes' rays, up to three steps per iteration (two: 1-2% slower, four:
@@ -406,7 +407,9 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
                     steps++;
                     const bool out = x < 0.0f || y < 0.0f || z < 0.0f || x >= wx || y >= wy || z >= wz || frac >= max_dist;
                     if (hit || out || steps >= max_steps) {
-                        end_ray(my, x, y, z, hit, (uint32_t)steps | (hit ? (1u << 24) : (out ? 0u : (1u << 25))));
+                        end_ray(my, x, y, z, hit,
+                                (uint32_t)steps | (fexit >= 0.0f && frac == f ? kInfoRegular : 0u) |
+                                    (hit ? kInfoHit : (out ? 0u : kInfoCapped)));
                         my = -1;
                         fin = true;
                     }
@@ -559,116 +562,159 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
 }
 
 // ---------------------------------------------------------------- finalize kernel
+// What a finalize CTA shares: its hits' ray numbers, every ray's light by channel and task
+// (kFinStride: 32 and one, so that lanes reading different tasks hit different banks), counters.
+constexpr int kFinStride = kTaskRays + 1;
+struct FinShared {
+    float light[3 * kFinWarps * kFinStride];
+    uint8_t hit[kFinWarps * kTaskRays];
+    int n_hits;
+    unsigned lookups;
+    __device__ __forceinline__ void put_light(int task, int lane, float3 v) {
+        float* s = light + task * kFinStride + lane;
+        s[0] = v.x;
+        s[kFinWarps * kFinStride] = v.y;
+        s[2 * kFinWarps * kFinStride] = v.z;
+    }
+};
+static_assert(kFinWarps * kTaskRays <= 256 && 3 * kFinWarps <= 32 && (kFinWarps & (kFinWarps - 1)) == 0,
+              "ray numbers fit 8 bits, one lane per channel and task");
+
+// Warps per CTA, and CTAs per SM of the lean and the general form.  The kernel waits on its chain of
+// dependent lookups and its barriers, so small CTAs pay: two warps for a group's eight tasks, 24 CTAs
+// per SM at 40 registers (44 B of spills).  On the demo's 8-pass step / a 64-ray demo frame / 64
+// worlds batched: 717 / 186 / 2,601 us; four warps 730 / 191 / 2,700; eight warps, one task each,
+// 725 / 197 / 2,775; two warps at 32 registers 836 / 196 / 2,649, at 48 registers 754 / 190 / 2,627;
+// one warp 793 / 190 / 2,648.
+constexpr int kFinCtaWarps = 2;
+constexpr int kFinLeanCtas = 24, kFinGeneralCtas = 16;
+// A launch of at most this many groups per SM has no second round of CTAs to keep the SMs busy: it
+// runs a warp per task (6 CTAs per SM), whose CTAs finish sooner.  One 64-ray pass of 79 / 306 / 832 /
+// 1,728 / 2,693 / 4,224 groups on 152 SMs: 20.7 / 25.6 / 31.0 / 44.7 / 55.5 / 73.7 us against 20.8 /
+// 32.4 / 36.8 / 46.5 / 55.4 / 73.5 us with two warps; the lines cross near 2,500.
+// The general form's warp-per-task CTAs run 4 to an SM: an R = 96 pass of 459 groups 28.6 against 32.8
+// us, of 1,570 groups 92.6 against 86.0.
+constexpr int kFinFewGroups = 16, kFinFewGeneral = 4;
+
+// One group of eight consecutive tasks (one CTA's work).  A warp per task in lock step had 20 of 32
+// lanes active: odd rays of a subgroup point the other way, so most tasks mix hits and misses.  Here
+// the CTA's hits are refined and shaded 32 to a warp, and one lane per task and channel sums the
+// subgroup in the butterfly's order from shared memory: 38.3 -> 28.1 M warp instructions per pass of
+// the demo step.
 // IN_CTA: every probe of the launch combines inside one CTA (R/32 divides kFinWarps); the kernel
-// then has no global-memory combine, which costs the general kernel 8 registers and spills.  The
-// kernel waits on its lookup chain, so occupancy pays: the lean forms run 8 CTAs per SM at 32
-// registers (the world-table form: 52 B of spills, the 256-world batch 2.8% faster than at 6 CTAs
-// and 40 registers; at 4 CTAs it was slower again: five 4-6% faster, six 1% faster), the
-// device loop's persistent form 6 (its spills at 32 registers would be 208 B).
-// One 8-task group (one CTA's work) of the finalize kernel.  SINGLE: the launch covers one world
-// (a single pass, or one pass of a several-pass call), read from the kernel's parameters, whose
-// fields are operands from the constant bank; else the world table's entry for the group through
-// a generic pointer, whose fields the compiler keeps in registers.  SINGLE took the lean kernel
-// from 40 registers and 24 B of spills to 40 registers and none (the 8-pass step 5.6% faster, a
-// single pass 2.8%), and then fits 8 CTAs per SM at 32 registers with 32 B of spills: 1.9% faster
-// again on the 8-pass step, 0.9% on a single pass (launch 48.8 against 51.0 us).
-template <class Store, bool RECORD, bool IN_CTA, bool SINGLE>
-__device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, float4* s_mean, int* s_count,
-                                               unsigned (*s_stat)[2]) {
+// then has no global-memory combine.  SINGLE: the launch covers one world (a single pass, or one
+// pass of a several-pass call), read from the kernel's parameters, whose fields are operands from
+// the constant bank; else the world table's entry for the group through a generic pointer.
+template <class Store, bool RECORD, bool IN_CTA, bool SINGLE, int CW>
+__device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, FinShared& sh) {
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
-    if (threadIdx.x < kFinWarps) {
-        s_count[threadIdx.x] = 0;
-        s_stat[threadIdx.x][0] = 0;
-        s_stat[threadIdx.x][1] = 0;
+    if (threadIdx.x == 0) {
+        sh.n_hits = 0;
+        sh.lookups = 0;
     }
     __syncthreads();
     const int t0 = la.chunk_begin + group * kFinWarps;   // worlds start at multiples of 8
-    const int t = t0 + w;
     const WorldPass* wp = SINGLE ? &la.single : la.worlds ? la.worlds + world_of(la, t0) : &la.single;
-    const int t_local = t - (int)wp->task_begin;
-    bool valid = t < la.chunk_end && t_local < wp->n_tasks;
+    const int t0_local = t0 - (int)wp->task_begin;
+    long long n_tasks = min(wp->n_tasks, (long long)la.chunk_end - wp->task_begin);
     if (la.dev_count)   // a list built on the device (single world): its own length bounds the tasks
-        valid = valid && t_local < (__ldcg(la.dev_count) / wp->size) * (wp->R >> 5);
-    const int nsub = wp->R >> 5;
-    const int g = div_nsub(max(t_local, 0), nsub);
-    const int k = t_local - g * nsub;
-    // a probe's subgroups share this CTA when R/32 divides 8 (task_begin is a multiple of 8)
-    const bool local = nsub > 1 && (kFinWarps % nsub) == 0 && (wp->task_begin % kFinWarps) == 0;
-    float3 v = make_float3(0.0f, 0.0f, 0.0f);
-    if (valid) {
-        const int idx = (t - la.ray_origin) * kTaskRays + lane;
-        const uint2 res = __ldcg(la.rays.res + idx);
-        const float4 od = __ldcg(la.rays.od + idx);
-        const float2 dd = __ldcg(la.rays.dd + idx);
-        const int blk = RECORD ? __ldcg(la.ray_blk + idx) : 0;
-        const float3 o = make_float3(od.x, od.y, od.z);
-        const float3 d = make_float3(od.w, dd.x, dd.y);
-        uint32_t lookups;
-        float3 L, u;
+        n_tasks = min(n_tasks, (long long)(__ldcg(la.dev_count) / wp->size) * (wp->R >> 5));
+    const int first = (t0 - la.ray_origin) * kTaskRays;   // the group's first ray in the ray buffer
+    // 1. the tasks' rays, one warp a task: the hits into the CTA's list, the misses' light.  (Every
+    // ray is read here, through L1: a hit's origin and direction then wait there for step 2.)
+    unsigned lookups = 0;
+#pragma unroll
+    for (int k = w; k < kFinWarps; k += CW) {
+        if (t0_local + k >= n_tasks) break;
+        const int idx = first + k * kTaskRays + lane;
+        const uint2 res = la.rays.res[idx];
+        const float2 dd = la.rays.dd[idx];
+        const float4 od = la.rays.od[idx];
+        const bool hit = res.y & kInfoHit;
+        lookups += res.y & 0xffffu;
+        const unsigned hm = __ballot_sync(kFull, hit);
+        int base = 0;
+        if (lane == 0 && hm) base = atomicAdd(&sh.n_hits, __popc(hm));
+        base = __shfl_sync(kFull, base, 0);
+        if (hit) {
+            sh.hit[base + __popc(hm & ((1u << lane) - 1u))] = (uint8_t)(k * kTaskRays + lane);
+        } else {
+            sh.put_light(k, lane, sky_light(make_float3(od.w, dd.x, dd.y)));
+            if (RECORD)
+                record_miss(*wp, __uint_as_float(res.x), res.y, __ldcg(la.ray_blk + idx), (long long)(t0_local + k) * kTaskRays + lane);
+        }
+    }
+    __syncthreads();
+    // 2. the hits, packed 32 to a warp (the first 32 to another warp in each group, so that every
+    // scheduler of the SM gets its share)
+    const int n_hits = sh.n_hits;
+#pragma unroll 1
+    for (int j = (int)(threadIdx.x + 32 * (group % CW)) % (32 * CW); j < n_hits; j += 32 * CW) {
+        const int ray = sh.hit[j], idx = first + ray;
+        const uint2 res = la.rays.res[idx];
+        const float4 od = la.rays.od[idx];
+        const float2 dd = la.rays.dd[idx];
+        const float3 o = make_float3(od.x, od.y, od.z), d = make_float3(od.w, dd.x, dd.y);
+        const float frac = __uint_as_float(res.x);
+        float3 u;
         float4 m;
-        const MarchView mv = march_view(*wp);
-        const float fc = __uint_as_float(res.x);
-        const long long gr = (long long)t_local * kTaskRays + lane;
-        const bool hit = mv.wide ? finalize_ray<RECORD, true>(*wp, mv, o, d, fc, res.y, blk, gr, lookups, L, u, m)
-                                 : finalize_ray<RECORD, false>(*wp, mv, o, d, fc, res.y, blk, gr, lookups, L, u, m);
+        if (RECORD) {
+            lookups += refine_general<true>(*wp, o, d, frac, res.y, __ldcg(la.ray_blk + idx), (long long)t0_local * kTaskRays + ray, u, m);
+        } else if (res.y & kInfoRegular) {
+            const MarchView mv = march_view(*wp);
+            lookups += mv.wide ? refine_regular<true>(*wp, mv, o, d, frac, u, m) : refine_regular<false>(*wp, mv, o, d, frac, u, m);
+        } else {
+            lookups += refine_irregular(*wp, o, d, frac, u, m);
+        }
         grid_dependency_wait();   // from here on the volumes: the previous pass's launch has finished
-        if (hit) L = shade_hit<Store>(*wp, u, m);
-        L = butterfly_sum(L);
-        v = make_float3(fmul(L.x, 0.03125f), fmul(L.y, 0.03125f), fmul(L.z, 0.03125f));   // /32
-        // counters: lookups and hits of this task, summed per CTA below
-        const unsigned a = __reduce_add_sync(kFull, lookups);
-        const unsigned h = __popc(__ballot_sync(kFull, (res.y >> 24) & 1u));
-        if (lane == 0) {
-            s_stat[w][0] = a;
-            s_stat[w][1] = h;
-            if (nsub == 1) {
-                store_probe<Store>(*wp, g, make_float3(fadd(0.0f, v.x), fadd(0.0f, v.y), fadd(0.0f, v.z)));
-            } else if (!local) {
-                if (IN_CTA) atomicOr(la.error, 2);   // launched with the wrong kernel: reported, never stored
-                else subgroup_done<Store>(*wp, g, k, v);
-            } else {
-                // the last of the probe's subgroups in this CTA sums their means in subgroup
-                // order (radiance.comp:401-407)
-                volatile float* vm = reinterpret_cast<volatile float*>(s_mean);
-                vm[4 * w] = v.x;
-                vm[4 * w + 1] = v.y;
-                vm[4 * w + 2] = v.z;
-                __threadfence_block();
-                if (atomicAdd(&s_count[w - k], 1) == nsub - 1) {
-                    __threadfence_block();
-                    float3 acc = make_float3(0.0f, 0.0f, 0.0f);
-                    for (int j = w - k; j < w - k + nsub; j++) {
-                        const float sx = vm[4 * j], sy = vm[4 * j + 1], sz = vm[4 * j + 2];
-                        acc = make_float3(fadd(acc.x, sx), fadd(acc.y, sy), fadd(acc.z, sz));
-                    }
-                    const float fn = (float)nsub;
-                    acc = make_float3(fdiv_by(acc.x, fn, wp->inv_nsub), fdiv_by(acc.y, fn, wp->inv_nsub),
-                                      fdiv_by(acc.z, fn, wp->inv_nsub));
-                    store_probe<Store>(*wp, g, acc);
-                }
-            }
+        sh.put_light(ray >> 5, ray & 31, shade_hit<Store>(*wp, u, m));
+    }
+    lookups = __reduce_add_sync(kFull, lookups);
+    if (lane == 0 && lookups) atomicAdd(&sh.lookups, lookups);
+    __syncthreads();
+    // 3. one warp: lane 8*c + k sums channel c of task k, then the tasks of a probe in order
+    if (w != group % CW) return;
+    const int k8 = lane & (kFinWarps - 1);
+    const int t_local = t0_local + k8;
+    const bool valid = lane < 3 * kFinWarps && t_local < n_tasks;
+    const float mean = valid ? fmul(butterfly_sum(sh.light + lane * kFinStride), 0.03125f) : 0.0f;   // /32
+    grid_dependency_wait();
+    const int nsub = wp->R >> 5;
+    // a probe's subgroups share this CTA when R/32 divides 8 (task_begin is a multiple of 8)
+    const bool local = (kFinWarps % nsub) == 0 && (wp->task_begin % kFinWarps) == 0;
+    float acc = mean;
+    if (local) {   // the subgroups' means summed in subgroup order (radiance.comp:401-407)
+        acc = 0.0f;
+        const int head = lane & ~(nsub - 1);
+        for (int i = 0; i < nsub; i++) acc = fadd(acc, __shfl_sync(kFull, mean, head + i));
+        acc = fdiv_by(acc, (float)nsub, wp->inv_nsub);
+    }
+    const float3 v = make_float3(acc, __shfl_sync(kFull, acc, kFinWarps + k8), __shfl_sync(kFull, acc, 2 * kFinWarps + k8));
+    if (lane < kFinWarps && valid) {
+        const int g = div_nsub(t_local, nsub);
+        const int k = t_local - g * nsub;
+        if (local) {
+            if (k == 0) store_probe<Store>(*wp, g, v);
+        } else if (IN_CTA) {
+            atomicOr(la.error, 2);   // launched with the wrong kernel: reported, never stored
+        } else {
+            subgroup_done<Store>(*wp, g, k, v);
         }
     }
     // the CTA's counters in one atomic each: one world per CTA; same-address atomics from every
     // task serialise at one L2 slice and held warps at exit (measured 5% of the pass)
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long a = 0, h = 0;
-        for (int j = 0; j < kFinWarps; j++) {
-            a += s_stat[j][0];
-            h += s_stat[j][1];
-        }
-        if (a) atomicAdd(wp->stats, a);
-        if (h) atomicAdd(wp->stats + 1, h);
+    if (lane == 0) {
+        if (sh.lookups) atomicAdd(wp->stats, (unsigned long long)sh.lookups);
+        if (sh.n_hits) atomicAdd(wp->stats + 1, (unsigned long long)sh.n_hits);
         if (la.time_end) atomicMax(la.time_end + 1, globaltimer_ns());
     }
 }
 
 // PERSIST (launches sized on the device): a fixed grid walks the 8-task groups of the device's
 // task count; otherwise one CTA per group.
-template <class Store, bool RECORD, bool IN_CTA, bool PERSIST = false, bool SINGLE = false>
-__global__ void __launch_bounds__(kFinWarps * 32, IN_CTA ? (PERSIST ? 6 : 8) : 4)
+template <class Store, bool RECORD, bool IN_CTA, bool PERSIST = false, bool SINGLE = false, int CW = kFinCtaWarps>
+__global__ void __launch_bounds__(CW * 32, (IN_CTA ? kFinLeanCtas : kFinGeneralCtas) * kFinCtaWarps / CW)
 finalize_kernel(const __grid_constant__ LaunchArgs la) {
     grid_launch_dependents();   // the next pass's launch may start its volume-free part
     if (la.pass_mask && (int)blockIdx.x >= la.fin_ctas) {   // copy role (see LaunchArgs)
@@ -687,18 +733,16 @@ finalize_kernel(const __grid_constant__ LaunchArgs la) {
         if (threadIdx.x == 0 && la.time_end) atomicMax(la.time_end + 1, globaltimer_ns());
         return;
     }
-    __shared__ float4 s_mean[kFinWarps];
-    __shared__ int s_count[kFinWarps];
-    __shared__ unsigned s_stat[kFinWarps][2];
+    __shared__ FinShared sh;
     if (!PERSIST) {
-        finalize_group<Store, RECORD, IN_CTA, SINGLE>(la, (int)blockIdx.x, s_mean, s_count, s_stat);
+        finalize_group<Store, RECORD, IN_CTA, SINGLE, CW>(la, (int)blockIdx.x, sh);
         return;
     }
     const long long total = la.dev_total ? __ldcg(la.dev_total) : (long long)la.chunk_end;
     const int groups = (int)((min(total, (long long)la.chunk_end) - la.chunk_begin + kFinWarps - 1) / kFinWarps);
     for (int g = (int)blockIdx.x; g < groups; g += (int)gridDim.x) {
-        finalize_group<Store, RECORD, IN_CTA, false>(la, g, s_mean, s_count, s_stat);
-        __syncthreads();   // thread 0 has read the counters before the next group clears them
+        finalize_group<Store, RECORD, IN_CTA, false, CW>(la, g, sh);
+        __syncthreads();   // the group's counters and light are read before the next group's
     }
 }
 
@@ -795,12 +839,19 @@ void launch_march(LaunchArgs args, const WorldPass& w, long long round_tasks, in
 // volume reads and writes wait for that kernel's end (griddepcontrol.wait).  single: every task of
 // the launch belongs to args.single.
 template <class Store, bool RECORD>
-void launch_finalize(const LaunchArgs& args, int n, bool in_cta, cudaStream_t stream, bool overlap, bool single) {
-    const int blocks = (n + kFinWarps - 1) / kFinWarps + (args.pass_mask ? args.fin_copy : 0);
+void launch_finalize(const LaunchArgs& args, int n, bool in_cta, cudaStream_t stream, bool overlap, bool single, int num_sms) {
+    const int groups = (n + kFinWarps - 1) / kFinWarps;
+    const int blocks = groups + (args.pass_mask ? args.fin_copy : 0);
     if (blocks <= 0) return;
+    if (!RECORD && groups <= (in_cta ? kFinFewGroups : kFinFewGeneral) * num_sms) {
+        auto k = single ? (in_cta ? finalize_kernel<Store, false, true, false, true, kFinWarps> : finalize_kernel<Store, false, false, false, true, kFinWarps>)
+                        : (in_cta ? finalize_kernel<Store, false, true, false, false, kFinWarps> : finalize_kernel<Store, false, false, false, false, kFinWarps>);
+        launch_k(k, blocks, kFinWarps * 32, 0, stream, overlap, args);
+        return;
+    }
     auto k = single ? (in_cta ? finalize_kernel<Store, RECORD, true, false, true> : finalize_kernel<Store, RECORD, false, false, true>)
                     : (in_cta ? finalize_kernel<Store, RECORD, true> : finalize_kernel<Store, RECORD, false>);
-    launch_k(k, blocks, kFinWarps * 32, 0, stream, overlap, args);
+    launch_k(k, blocks, kFinCtaWarps * 32, 0, stream, overlap, args);
 }
 
 template <class Store, bool RECORD>
@@ -821,7 +872,7 @@ cudaError_t launch_t(const LaunchArgs& a, int num_sms, cudaStream_t stream, bool
         args.count_dst = nullptr;
         args.time_start = nullptr;
         const bool lean = a.force_lean || (a.worlds ? a.in_cta != 0 : combines_in_cta(&a.single, 1));
-        launch_finalize<Store, RECORD>(args, n, lean, stream, false, a.worlds == nullptr);
+        launch_finalize<Store, RECORD>(args, n, lean, stream, false, a.worlds == nullptr, num_sms);
     }
     return cudaGetLastError();
 }
@@ -849,7 +900,7 @@ cudaError_t passes_t(const LaunchArgs& a, const WorldPass* h_tab, int n_passes, 
     args.time_start = nullptr;
     const bool in_cta = combines_in_cta(h_tab, n_passes);
     const long long probes = (long long)(vol_bytes / sizeof(typename Store::T));
-    const int copy_ctas = (int)std::max<long long>(1, std::min<long long>((probes + 1023) / 1024, 2LL * num_sms));
+    const int copy_ctas = (int)std::max<long long>(1, std::min<long long>((probes + 255) / 256, 8LL * num_sms));
     for (int i = 0; i < n_passes; i++) {
         const WorldPass& w = h_tab[i];
         args.chunk_begin = (int)w.task_begin;
@@ -865,7 +916,7 @@ cudaError_t passes_t(const LaunchArgs& a, const WorldPass* h_tab, int n_passes, 
         args.single = w;   // the launch's tasks are pass i's
         // from the second pass on, the launch overlaps the previous pass's tail: its refine and
         // materials read no volume (the first pass's rays come from the march launch before it)
-        launch_finalize<Store, false>(args, n, in_cta, stream, i > 0, true);
+        launch_finalize<Store, false>(args, n, in_cta, stream, i > 0, true, num_sms);
     }
     return cudaGetLastError();
 }
@@ -896,14 +947,14 @@ cudaError_t launch_table_pass(const LaunchArgs& a, int precision, int num_sms, c
     // mostly small (p50 5-8% lower at 2,000-10,000 requests/s than the per-warp queue; 2% less
     // throughput saturated, where the host loop is the faster one anyway)
     march_kernel<false, false, true><<<blocks, kWarps * 32, 0, stream>>>(args);
-    const int fin = num_sms * 6;   // the persistent finalize's occupancy (6 CTAs per SM)
+    const int fin = num_sms * kFinLeanCtas;
     switch (precision) {
-        case LUMRAD_PRECISION_FP16: finalize_kernel<StoreF16, false, true, true><<<fin, kFinWarps * 32, 0, stream>>>(args); break;
-        case LUMRAD_PRECISION_BF16: finalize_kernel<StoreBF16, false, true, true><<<fin, kFinWarps * 32, 0, stream>>>(args); break;
+        case LUMRAD_PRECISION_FP16: finalize_kernel<StoreF16, false, true, true><<<fin, kFinCtaWarps * 32, 0, stream>>>(args); break;
+        case LUMRAD_PRECISION_BF16: finalize_kernel<StoreBF16, false, true, true><<<fin, kFinCtaWarps * 32, 0, stream>>>(args); break;
         case LUMRAD_PRECISION_RGB10A2:
-            finalize_kernel<StoreRGB10A2, false, true, true><<<fin, kFinWarps * 32, 0, stream>>>(args);
+            finalize_kernel<StoreRGB10A2, false, true, true><<<fin, kFinCtaWarps * 32, 0, stream>>>(args);
             break;
-        default: finalize_kernel<StoreF32, false, true, true><<<fin, kFinWarps * 32, 0, stream>>>(args);
+        default: finalize_kernel<StoreF32, false, true, true><<<fin, kFinCtaWarps * 32, 0, stream>>>(args);
     }
     return cudaGetLastError();
 }
@@ -1188,8 +1239,7 @@ extern "C" int lumrad_radiance_pass_noalloc(const int* world_size, const int16_t
     w.one_minus_alpha = 1.0f - p->blend;
     w.seed = (uint32_t)p->time_seed;
     for (int i = 0; i < 3; i++) {
-        const int v = world_size[i];
-        w.inv_dim[i] = (v & (v - 1)) == 0 ? 1.0f / (float)v : 0.0f;
+        w.inv_dim[i] = 1.0f / (float)world_size[i];
     }
     w.inv_nsub = 1.0f / (float)(R / 32);
     w.dirs = dirs;
@@ -1210,7 +1260,7 @@ extern "C" int lumrad_radiance_pass_noalloc(const int* world_size, const int16_t
         const int tasks = la.chunk_end - la.chunk_begin;
         if (tasks < kCtaQueueTasksPerWarp * la.total_warps) march_kernel<false, false, true><<<blocks, kWarps * 32, 0, stream>>>(la);
         else march_kernel<false><<<blocks, kWarps * 32, 0, stream>>>(la);
-        finalize_kernel<StoreF32, false, true, false, true><<<(tasks + kFinWarps - 1) / kFinWarps, kFinWarps * 32, 0, stream>>>(la);
+        finalize_kernel<StoreF32, false, true, false, true><<<(tasks + kFinWarps - 1) / kFinWarps, kFinCtaWarps * 32, 0, stream>>>(la);
     }
     LUMRAD_TRY(cudaGetLastError());
     return LUMRAD_OK;
