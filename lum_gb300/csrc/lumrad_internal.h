@@ -18,8 +18,8 @@ constexpr int kTaskRays = 32;
 // tasks' rays (32 B per ray: 268 MB).  Fewer, larger rounds shorten the march kernel's tails
 // (measured: 2^18 tasks 13% faster than 2^16 on many small worlds).
 constexpr int kChunkTasks = 1 << 18;
-// Words of a launch's task queue: [0] next march task, [1] march warps finished; zero between
-// launches (the march's last warp resets them)
+// Words of a launch's task queue: [0] next march task, [1] march CTAs finished; zero between
+// launches (the march's last CTA resets them)
 constexpr int kQueueWords = 2;
 // Round size of batches: their task spaces are large, and two rounds of 2^20 tasks beat seven of
 // 2^18 by 2% on 256 mixed worlds (fewer queue drains; measured with 8-byte ray results)
