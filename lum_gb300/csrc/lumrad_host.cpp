@@ -462,7 +462,8 @@ int Context::run_pass(const short4* d_reqs, int n, const LumRadPassParams* p_in,
     if ((rc = ensure_rays(la.n_tasks))) return rc;
     // the march may start in the previous pass's finalize tail: see pass_mark (the list must not
     // come from a kernel, the hits use the one record buffer)
-    const bool dependent = !p.record_hits && !dev_count && pass_mark == api_calls - 1 && uploads_mark == world.uploads;
+    // (over a device list it waits for the list's kernels before it reads anything of theirs)
+    const bool dependent = !p.record_hits && (dev_count || (pass_mark == api_calls - 1 && uploads_mark == world.uploads));
     la.rays = ray_buffer(d_rays[ray_side], ray_cap);
     ray_side ^= 1;
     la.ray_blk = d_ray_blk;

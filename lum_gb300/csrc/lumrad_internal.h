@@ -142,6 +142,10 @@ struct LaunchArgs {
     // would keep the next pass's march from starting in the previous finalize's tail.)
     unsigned long long* time_start;
     unsigned long long* time_end;
+    // the finalize launch is a programmatic dependent of the march that wrote its rays: it waits for
+    // that launch first (else before its first volume access), and lets its own dependents start
+    // only then
+    int after_march;
     // scheduling (0 = the kernel's defaults, 2 and 32): a warp claims remaining / (guided_div *
     // warps) tasks at a time, clamped to [1, max_chunk]; the march grid has march_ctas CTAs per SM
     // (capped by occupancy)

@@ -3,8 +3,9 @@
 //   update list   the probes update_radiance relights each frame (internal_render.cpp:1142-1168):
 //                 every block whose clamped 3x3x3 neighbourhood has a positive id sum, in scan
 //                 order, then each special request whose block is not already listed, in request
-//                 order.  Four launches: flag (one bit per block, ballot) + per-CTA counts, a
-//                 single-CTA scan of the counts, an order-preserving write, and the specials.
+//                 order.  Two launches: flag (one bit per block, ballot) + per-CTA counts, and an
+//                 order-preserving write; a scan of the counts between them for worlds of more than a
+//                 million blocks, and a third launch when there are specials.
 //   scroll        shift_radiance (internal_render.cpp:1218-1335): new(p) = old(p + shift) where
 //                 p + shift is inside the world, old(p) elsewhere; one pass into the other
 //                 ping-pong volume.
@@ -16,6 +17,7 @@
 // contraction), so results are reproducible bit for bit.
 
 #include "radiance_device.cuh"
+#include "lumrad_launch.h"
 
 #include <algorithm>
 
@@ -27,36 +29,44 @@ constexpr int kScanCta = 1024;
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
+// The list kernels are bound by launch latency (a few us each, about 1 us of work at 65,536 blocks): two
+// launches instead of four, and the frame's kernels (scroll, list, march, finalize of few groups,
+// gather) each a programmatic dependent of the one before.  A lone 8x8x8 / 19x38x9 / 45x38x11 frame:
+// 39.6 / 57.2 / 81.2 -> 22.6 / 38.8 / 62.8 us.
+//
+// The flags and counts (the grid does not come from a kernel: they are formed while the stream's
+// previous kernel still runs, then this one waits for it; see launch_kernel).
 __global__ void __launch_bounds__(kListCta)
-list_flags_kernel(const int16_t* __restrict__ grid, int X, int Y, int Z, long long W, uint32_t* __restrict__ bits,
+list_flags_kernel(const int16_t* __restrict__ grid, int X, int Y, int Z, unsigned W, uint32_t* __restrict__ bits,
                   int* __restrict__ cta_counts) {
+    grid_launch_dependents();
     __shared__ int s_cnt[kListCta / 32];
-    const long long i = (long long)blockIdx.x * kListCta + threadIdx.x;
+    const unsigned i = blockIdx.x * kListCta + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     bool flag = false;
     if (i < W) {
-        const int x = (int)(i % X);
-        const long long q = i / X;
-        const int y = (int)(q % Y);
-        const int z = (int)(q / Y);
+        const unsigned q = i / (unsigned)X;
+        const int x = (int)(i - q * X), z = (int)(q / (unsigned)Y), y = (int)(q - (unsigned)z * Y);
+        const int xs[3] = {max(x - 1, 0), x, min(x + 1, X - 1)};
         int sum = 0;   // sum of the 27 clamped neighbours' ids (internal_render.cpp:1147-1156)
+#pragma unroll
         for (int dz = -1; dz <= 1; dz++) {
             const int tz = clampi(z + dz, 0, Z - 1);
+#pragma unroll
             for (int dy = -1; dy <= 1; dy++) {
                 const int ty = clampi(y + dy, 0, Y - 1);
                 const int16_t* row = grid + (size_t)X * ((size_t)ty + (size_t)Y * tz);
-                for (int dx = -1; dx <= 1; dx++) sum += __ldg(row + clampi(x + dx, 0, X - 1));
+#pragma unroll
+                for (int k = 0; k < 3; k++) sum += __ldg(row + xs[k]);
             }
         }
         flag = sum > 0;
     }
     const unsigned b = __ballot_sync(kFull, flag);
-    const long long word = i >> 5;
-    if (lane == 0) {
-        if (word < (W + 31) / 32) bits[word] = b;
-        s_cnt[warp] = __popc(b);
-    }
+    if (lane == 0) s_cnt[warp] = __popc(b);
     __syncthreads();
+    grid_dependency_wait();
+    if (lane == 0 && i < W) bits[i >> 5] = b;
     if (threadIdx.x == 0) {
         int c = 0;
         for (int w = 0; w < kListCta / 32; w++) c += s_cnt[w];
@@ -106,26 +116,56 @@ list_scan_kernel(const int* __restrict__ counts, int n, int* __restrict__ offset
     if (threadIdx.x == 0) *total = carry;
 }
 
+// The list from the bits.  A CTA's offset: offsets[blockIdx.x] of a scan of the counts, or, with
+// offsets null (up to kDirectCtas CTAs), the sum of the counts before its own, formed here; the last
+// CTA then also writes the length.
+constexpr int kDirectCtas = 4096;
 __global__ void __launch_bounds__(kListCta)
-list_write_kernel(const uint32_t* __restrict__ bits, const int* __restrict__ offsets, int X, int Y, long long W,
-                  short4* __restrict__ out) {
-    __shared__ int s_pre[kListCta / 32];
-    const long long words = (W + 31) / 32;
-    if (threadIdx.x < kListCta / 32) {
-        const long long wi = (long long)blockIdx.x * (kListCta / 32) + threadIdx.x;
-        s_pre[threadIdx.x] = wi < words ? __popc(bits[wi]) : 0;
+list_write_kernel(const uint32_t* __restrict__ bits, const int* __restrict__ counts, const int* __restrict__ offsets, int X,
+                  int Y, unsigned W, short4* __restrict__ out, int* __restrict__ total, int* __restrict__ total2) {
+    grid_launch_dependents();
+    __shared__ int s_pre[kListCta / 32], s_sum[kListCta / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned i = blockIdx.x * kListCta + threadIdx.x;
+    const unsigned q = i / (unsigned)X, z = q / (unsigned)Y;
+    grid_dependency_wait();
+    const uint32_t b = i < W ? __ldcg(bits + (i >> 5)) : 0u;
+    int sum = 0;
+    if (!offsets)
+        for (int c = threadIdx.x; c < (int)blockIdx.x; c += kListCta) sum += __ldcg(counts + c);
+    sum = __reduce_add_sync(kFull, sum);
+    if (lane == 0) {
+        s_pre[warp] = __popc(b);
+        s_sum[warp] = sum;
     }
     __syncthreads();
-    const long long i = (long long)blockIdx.x * kListCta + threadIdx.x;
-    if (i >= W) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t b = bits[i >> 5];
+    int pos = offsets ? offsets[blockIdx.x] : 0, all = 0;
+    for (int w = 0; w < kListCta / 32; w++) {
+        pos += s_sum[w] + (w < warp ? s_pre[w] : 0);
+        all += s_pre[w];
+    }
+    if (total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        *total = pos + all;
+        if (total2) *total2 = pos + all;
+    }
     if (!((b >> lane) & 1u)) return;
-    int pos = offsets[blockIdx.x] + __popc(b & ((1u << lane) - 1u));
-    for (int w = 0; w < warp; w++) pos += s_pre[w];
-    const int x = (int)(i % X);
-    const long long q = i / X;
-    out[pos] = make_short4((short)x, (short)(q % Y), (short)(q / Y), 0);
+    out[pos + __popc(b & ((1u << lane) - 1u))] = make_short4((short)(i - q * X), (short)(q - z * Y), (short)z, 0);
+}
+
+// Launches of the list from bits and counts: the length into *total (and *total2 if not null).
+cudaError_t launch_list_write(const ListScratch& s, int X, int Y, long long W, short4* out, int* total, int* total2,
+                              cudaStream_t stream) {
+    const int ctas = (int)((W + kListCta - 1) / kListCta);
+    if (ctas <= kDirectCtas)
+        return launch_kernel(list_write_kernel, ctas, kListCta, 0, stream, true, s.bits, s.cta_counts, nullptr, X, Y, (unsigned)W,
+                             out, total, total2);
+    list_scan_kernel<<<1, kScanCta, 0, stream>>>(s.cta_counts, ctas, s.cta_offsets, total);
+    if (total2) {
+        const cudaError_t e = cudaMemcpyAsync(total2, total, sizeof(int), cudaMemcpyDeviceToDevice, stream);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_kernel(list_write_kernel, ctas, kListCta, 0, stream, false, s.bits, s.cta_counts, s.cta_offsets, X, Y,
+                         (unsigned)W, out, nullptr, nullptr);
 }
 
 // Dirty probes of block edits (Chebyshev distance <= r): a byte mask of the edited blocks, dilated
@@ -207,10 +247,11 @@ list_specials_kernel(const short4* __restrict__ sp, int ns, const uint32_t* __re
 template <typename V>
 __global__ void shift_kernel(const V* __restrict__ src, V* __restrict__ dst, int X, int Y, int Z, int sx, int sy,
                              int sz, long long W) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < W; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % X);
-        const long long q = i / X;
-        const int y = (int)(q % Y), z = (int)(q / Y);
+        const unsigned q = (unsigned)i / (unsigned)X;
+        const int x = (int)((unsigned)i - q * X), z = (int)(q / (unsigned)Y), y = (int)(q - (unsigned)z * Y);
         const int qx = x + sx, qy = y + sy, qz = z + sz;
         const bool inside = qx >= 0 && qx < X && qy >= 0 && qy < Y && qz >= 0 && qz < Z;
         dst[i] = inside ? src[(size_t)qx + (size_t)X * ((size_t)qy + (size_t)Y * qz)] : src[i];
@@ -364,6 +405,8 @@ __global__ void __launch_bounds__(kGatherCta)
 gather_kernel(const typename Store::T* __restrict__ rad, int X, int Y, int Z, const float* __restrict__ pts, int n,
               float* __restrict__ out) {
     __shared__ __align__(16) float s_buf[6 * kGatherCta];
+    grid_launch_dependents();
+    grid_dependency_wait();
     constexpr int kW = sizeof(V) / sizeof(float);
     const int first = blockIdx.x * kGatherCta, here = min(kGatherCta, n - first);
     const float* in = pts + 6 * (size_t)first;
@@ -529,10 +572,10 @@ cudaError_t launch_update_list(const int16_t* grid, int X, int Y, int Z, const s
                                const ListScratch& s, short4* out, int* count, cudaStream_t stream) {
     const long long W = (long long)X * Y * Z;
     const int ctas = (int)((W + kListCta - 1) / kListCta);
-    list_flags_kernel<<<ctas, kListCta, 0, stream>>>(grid, X, Y, Z, W, s.bits, s.cta_counts);
-    list_scan_kernel<<<1, kScanCta, 0, stream>>>(s.cta_counts, ctas, s.cta_offsets, s.listed);
-    list_write_kernel<<<ctas, kListCta, 0, stream>>>(s.bits, s.cta_offsets, X, Y, W, out);
-    list_specials_kernel<<<1, kScanCta, 0, stream>>>(specials, n_specials, s.bits, X, Y, s.listed, out, count);
+    cudaError_t e = launch_kernel(list_flags_kernel, ctas, kListCta, 0, stream, true, grid, X, Y, Z, (unsigned)W, s.bits, s.cta_counts);
+    if (e != cudaSuccess) return e;
+    if ((e = launch_list_write(s, X, Y, W, out, count, n_specials > 0 ? s.listed : nullptr, stream)) != cudaSuccess) return e;
+    if (n_specials > 0) list_specials_kernel<<<1, kScanCta, 0, stream>>>(specials, n_specials, s.bits, X, Y, s.listed, out, count);
     return cudaGetLastError();
 }
 
@@ -547,9 +590,7 @@ cudaError_t launch_dirty_list(const short4* edits, int n_edits, int X, int Y, in
     dirty_dilate_kernel<<<blocks, 256, 0, stream>>>(mask_a, mask_b, X, Y, Z, 0, radius, W);
     dirty_dilate_kernel<<<blocks, 256, 0, stream>>>(mask_b, mask_a, X, Y, Z, 1, radius, W);
     dirty_flags_kernel<<<ctas, kListCta, 0, stream>>>(mask_a, X, Y, Z, radius, W, s.bits, s.cta_counts);
-    list_scan_kernel<<<1, kScanCta, 0, stream>>>(s.cta_counts, ctas, s.cta_offsets, count);
-    list_write_kernel<<<ctas, kListCta, 0, stream>>>(s.bits, s.cta_offsets, X, Y, W, out);
-    return cudaGetLastError();
+    return launch_list_write(s, X, Y, W, out, count, nullptr, stream);
 }
 
 size_t list_scratch_words(long long W) { return (size_t)((W + 31) / 32); }
@@ -560,37 +601,33 @@ cudaError_t launch_shift_radiance(const void* src, void* dst, int X, int Y, int 
     const long long W = (long long)X * Y * Z;
     const int blocks = (int)std::min<long long>((W + 255) / 256, 152LL * 16);
     if (precision == LUMRAD_PRECISION_FP32)
-        shift_kernel<uint4><<<blocks, 256, 0, stream>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), X, Y,
-                                                        Z, sx, sy, sz, W);
-    else if (precision == LUMRAD_PRECISION_RGB10A2)
-        shift_kernel<unsigned><<<blocks, 256, 0, stream>>>(static_cast<const unsigned*>(src), static_cast<unsigned*>(dst),
-                                                           X, Y, Z, sx, sy, sz, W);
-    else
-        shift_kernel<uint2><<<blocks, 256, 0, stream>>>(static_cast<const uint2*>(src), static_cast<uint2*>(dst), X, Y,
-                                                        Z, sx, sy, sz, W);
-    return cudaGetLastError();
+        return launch_kernel(shift_kernel<uint4>, blocks, 256, 0, stream, true, static_cast<const uint4*>(src),
+                             static_cast<uint4*>(dst), X, Y, Z, sx, sy, sz, W);
+    if (precision == LUMRAD_PRECISION_RGB10A2)
+        return launch_kernel(shift_kernel<unsigned>, blocks, 256, 0, stream, true, static_cast<const unsigned*>(src),
+                             static_cast<unsigned*>(dst), X, Y, Z, sx, sy, sz, W);
+    return launch_kernel(shift_kernel<uint2>, blocks, 256, 0, stream, true, static_cast<const uint2*>(src),
+                         static_cast<uint2*>(dst), X, Y, Z, sx, sy, sz, W);
 }
 
 template <class Store>
-static void launch_gather_t(const void* rad, int X, int Y, int Z, const float* pts, int n, float* out, cudaStream_t stream) {
+static cudaError_t launch_gather_t(const void* rad, int X, int Y, int Z, const float* pts, int n, float* out, cudaStream_t stream) {
     const int blocks = (n + kGatherCta - 1) / kGatherCta;
     const typename Store::T* r = static_cast<const typename Store::T*>(rad);
     if (((reinterpret_cast<uintptr_t>(pts) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
-        gather_kernel<Store, float4><<<blocks, kGatherCta, 0, stream>>>(r, X, Y, Z, pts, n, out);
-    else
-        gather_kernel<Store, float><<<blocks, kGatherCta, 0, stream>>>(r, X, Y, Z, pts, n, out);
+        return launch_kernel(gather_kernel<Store, float4>, blocks, kGatherCta, 0, stream, true, r, X, Y, Z, pts, n, out);
+    return launch_kernel(gather_kernel<Store, float>, blocks, kGatherCta, 0, stream, true, r, X, Y, Z, pts, n, out);
 }
 
 cudaError_t launch_gather(const void* rad, int X, int Y, int Z, int precision, const float* pts, int n, float* out,
                           cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
     switch (precision) {
-        case LUMRAD_PRECISION_FP16: launch_gather_t<StoreF16>(rad, X, Y, Z, pts, n, out, stream); break;
-        case LUMRAD_PRECISION_BF16: launch_gather_t<StoreBF16>(rad, X, Y, Z, pts, n, out, stream); break;
-        case LUMRAD_PRECISION_RGB10A2: launch_gather_t<StoreRGB10A2>(rad, X, Y, Z, pts, n, out, stream); break;
-        default: launch_gather_t<StoreF32>(rad, X, Y, Z, pts, n, out, stream);
+        case LUMRAD_PRECISION_FP16: return launch_gather_t<StoreF16>(rad, X, Y, Z, pts, n, out, stream);
+        case LUMRAD_PRECISION_BF16: return launch_gather_t<StoreBF16>(rad, X, Y, Z, pts, n, out, stream);
+        case LUMRAD_PRECISION_RGB10A2: return launch_gather_t<StoreRGB10A2>(rad, X, Y, Z, pts, n, out, stream);
+        default: return launch_gather_t<StoreF32>(rad, X, Y, Z, pts, n, out, stream);
     }
-    return cudaGetLastError();
 }
 
 }  // namespace lumrad

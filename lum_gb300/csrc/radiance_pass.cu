@@ -36,6 +36,7 @@
 
 #include "radiance_device.cuh"
 #include "lumrad_devloop.h"
+#include "lumrad_launch.h"
 
 #include <type_traits>
 
@@ -188,10 +189,7 @@ __device__ __noinline__ long long refill_block(const LaunchArgs& la, int n_round
 template <bool RECORD, bool STAGE = false, bool CTAQ = false>
 __global__ void __launch_bounds__(STAGE ? kStageWarps * 32 : kWarps * 32, STAGE ? 1 : 4)
 march_kernel(const __grid_constant__ LaunchArgs la) {
-    if (la.time_start && blockIdx.x == 0 && threadIdx.x == 0) {   // the pass's kernel-time start
-        la.time_start[0] = globaltimer_ns();
-        la.time_start[1] = 0;
-    }
+    if (CTAQ) grid_launch_dependents();   // its finalize (LaunchArgs::after_march)
     if (la.pass_mask) {   // several passes: mark each pass's probes (this call's mask: the previous
                           // call's last finalize clears the other)
         const long long stride = (long long)gridDim.x * blockDim.x;
@@ -233,6 +231,11 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
         s_park = a_park;
     }
 
+    if (la.dev_count) grid_dependency_wait();   // a list from the kernels before (the world is in place by now)
+    if (la.time_start && blockIdx.x == 0 && threadIdx.x == 0) {   // the pass's kernel-time start
+        la.time_start[0] = globaltimer_ns();
+        la.time_start[1] = 0;
+    }
     int n_round = la.chunk_end - la.chunk_begin;
     if (la.dev_count) {   // a list built on the device: its own length bounds the round
         const long long real = (long long)(__ldcg(la.dev_count) / la.single.size) * (la.single.R >> 5);
@@ -736,6 +739,7 @@ __device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, 
 template <class Store, bool RECORD, bool IN_CTA, bool PERSIST = false, bool SINGLE = false, int CW = kFinCtaWarps>
 __global__ void __launch_bounds__(CW * 32, (IN_CTA ? kFinLeanCtas : kFinGeneralCtas) * kFinCtaWarps / CW)
 finalize_kernel(const __grid_constant__ LaunchArgs la) {
+    if (la.after_march) grid_dependency_wait();
     grid_launch_dependents();   // the next pass's launch may start its volume-free part
     if (la.pass_mask && (int)blockIdx.x >= la.fin_ctas) {   // copy role (see LaunchArgs)
         grid_dependency_wait();
@@ -809,47 +813,35 @@ size_t stage_bytes(const WorldPass& w) {
     return bytes <= (size_t)max_optin[dev] ? bytes : 0;
 }
 
-// A launch of `kern`; dependent: as a programmatic dependent of the stream's previous kernel (it
-// may start once every CTA of that kernel has called grid_launch_dependents; its reads and writes of
-// that kernel's data wait in grid_dependency_wait).
-cudaError_t launch_k(void (*kern)(LaunchArgs), int blocks, int threads, size_t smem, cudaStream_t stream, bool dependent,
-                     const LaunchArgs& args) {
-    if (!dependent) {
-        kern<<<blocks, threads, smem, stream>>>(args);
-        return cudaGetLastError();
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args);
-}
-
 // The march launch of a round (no hit records): staged when the world fits shared memory; the
-// CTA queue when the round has few tasks per warp.  dependent: see launch_k (the previous kernel
-// is the previous pass's finalize; the march writes the other ray buffer).
-void launch_march(LaunchArgs args, const WorldPass& w, long long round_tasks, int num_sms, cudaStream_t stream,
+// CTA queue when the round has few tasks per warp.  dependent: see launch_kernel (the previous kernel
+// is the previous pass's finalize, and the march writes the other ray buffer; or the list's, and the
+// march waits for it before it reads the list).  Returns whether it took the CTA queue: its finalize
+// may then be its programmatic dependent.
+bool launch_march(LaunchArgs args, const WorldPass& w, long long round_tasks, int num_sms, cudaStream_t stream,
                   bool dependent = false) {
     const size_t smem = stage_bytes(w);
     if (smem > 0) {
         const int blocks = (int)std::min<long long>(num_sms, std::max(round_tasks, 1LL));
         args.total_warps = blocks * kStageWarps;
         const bool q = round_tasks < (long long)kCtaQueueTasksPerWarp * args.total_warps;
-        launch_k(q ? march_kernel<false, true, true> : march_kernel<false, true>, blocks, kStageWarps * 32, smem, stream,
-                 dependent, args);
-    } else {
-        const int blocks = march_grid(false, num_sms, round_tasks, args.march_ctas);
-        args.total_warps = blocks * kWarps;
-        const bool q = round_tasks < (long long)kCtaQueueTasksPerWarp * args.total_warps;
-        launch_k(q ? march_kernel<false, false, true> : march_kernel<false>, blocks, kWarps * 32, 0, stream, dependent,
-                 args);
+        launch_kernel(q ? march_kernel<false, true, true> : march_kernel<false, true>, blocks, kStageWarps * 32, smem, stream,
+                      dependent, args);
+        return q;
     }
+    const int blocks = march_grid(false, num_sms, round_tasks, args.march_ctas);
+    args.total_warps = blocks * kWarps;
+    const bool q = round_tasks < (long long)kCtaQueueTasksPerWarp * args.total_warps;
+    launch_kernel(q ? march_kernel<false, false, true> : march_kernel<false>, blocks, kWarps * 32, 0, stream, dependent, args);
+    return q;
+}
+
+// Whether a finalize launch of n tasks is one of few groups (kFinFewGroups): a warp per task, and a
+// programmatic dependent of its march (8x8x8 / 20x20x8 / 32x32x12 blocks, 64 rays, a pass 16.5 / 20.6 /
+// 42.9 -> 11.4 / 19.0 / 40.1 us; with more groups the waiting CTAs are in the way of the march's end:
+// the 64-ray demo frame 181.3 us without, 185.4 with).
+bool few_groups(int n, bool in_cta, int num_sms) {
+    return (n + kFinWarps - 1) / kFinWarps <= (in_cta ? kFinFewGroups : kFinFewGeneral) * num_sms;
 }
 
 // overlap: launched as a programmatic dependent of the stream's previous kernel (a finalize launch
@@ -861,15 +853,15 @@ void launch_finalize(const LaunchArgs& args, int n, bool in_cta, cudaStream_t st
     const int groups = (n + kFinWarps - 1) / kFinWarps;
     const int blocks = groups + (args.pass_mask ? args.fin_copy : 0);
     if (blocks <= 0) return;
-    if (!RECORD && groups <= (in_cta ? kFinFewGroups : kFinFewGeneral) * num_sms) {
+    if (!RECORD && few_groups(n, in_cta, num_sms)) {
         auto k = single ? (in_cta ? finalize_kernel<Store, false, true, false, true, kFinWarps> : finalize_kernel<Store, false, false, false, true, kFinWarps>)
                         : (in_cta ? finalize_kernel<Store, false, true, false, false, kFinWarps> : finalize_kernel<Store, false, false, false, false, kFinWarps>);
-        launch_k(k, blocks, kFinWarps * 32, 0, stream, overlap, args);
+        launch_kernel(k, blocks, kFinWarps * 32, 0, stream, overlap, args);
         return;
     }
     auto k = single ? (in_cta ? finalize_kernel<Store, RECORD, true, false, true> : finalize_kernel<Store, RECORD, false, false, true>)
                     : (in_cta ? finalize_kernel<Store, RECORD, true> : finalize_kernel<Store, RECORD, false>);
-    launch_k(k, blocks, kFinCtaWarps * 32, 0, stream, overlap, args);
+    launch_kernel(k, blocks, kFinCtaWarps * 32, 0, stream, overlap, args);
 }
 
 template <class Store, bool RECORD>
@@ -883,14 +875,17 @@ cudaError_t launch_t(const LaunchArgs& a, int num_sms, cudaStream_t stream, bool
         args.chunk_end = (int)min(c0 + round, a.n_tasks);
         args.ray_origin = args.chunk_begin;
         const int n = args.chunk_end - args.chunk_begin;
+        bool queue = false;
         if (RECORD) march_kernel<RECORD><<<blocks, kWarps * 32, 0, stream>>>(args);
-        else launch_march(args, a.single, std::min(a.n_tasks, round), num_sms, stream, dependent && c0 == 0);
+        else queue = launch_march(args, a.single, std::min(a.n_tasks, round), num_sms, stream, dependent && c0 == 0);
         args.copy_dst = nullptr;   // the pass's start: in the first round's march only
         args.clear_stats = nullptr;
         args.count_dst = nullptr;
         args.time_start = nullptr;
         const bool lean = a.force_lean || (a.worlds ? a.in_cta != 0 : combines_in_cta(&a.single, 1));
-        launch_finalize<Store, RECORD>(args, n, lean, stream, false, a.worlds == nullptr, num_sms);
+        queue = queue && few_groups(n, lean, num_sms);
+        args.after_march = queue ? 1 : 0;
+        launch_finalize<Store, RECORD>(args, n, lean, stream, queue, a.worlds == nullptr, num_sms);
     }
     return cudaGetLastError();
 }
