@@ -17,6 +17,8 @@
 
 #include "lumrad_world.h"
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -735,7 +737,6 @@ void Context::release() {
     cudaFree(d_dirty_mask);
     cudaFree(d_edits);
     cudaFree(d_gather);
-    cudaFree(d_rgb);
     if (h_rgb) cudaFreeHost(h_rgb);
     for (auto& m : models) cudaFree(m.d_vox);
     models.clear();
@@ -938,20 +939,54 @@ static bool host_pinned(const void* p, size_t bytes) {
     return true;
 }
 
+// The device address of [p, p + bytes) if it lies in one page-locked host allocation or registration
+// the GPU can write, else null.
+static void* pinned_device_range(void* p, size_t bytes) {
+    typedef CUresult (*Attributes)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Attributes attributes = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Attributes>(f);
+    }();
+    if (!attributes) return nullptr;
+    // (an attribute that does not apply to the pointer is set to zero)
+    unsigned type = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    void* host = nullptr;
+    CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                   CU_POINTER_ATTRIBUTE_HOST_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* out[] = {&type, &dev, &host, &start, &size};
+    if (attributes(5, which, out, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return nullptr;
+    if (type != CU_MEMORYTYPE_HOST || !dev || host != p || size < bytes) return nullptr;
+    // the range starts at or before the pointer, by its host or its device address
+    const CUdeviceptr h = reinterpret_cast<CUdeviceptr>(p);
+    const bool by_host = h >= start && h - start <= size - bytes, by_dev = dev >= start && dev - start <= size - bytes;
+    return by_host || by_dev ? reinterpret_cast<void*>(dev) : nullptr;
+}
+
 int lumrad_get_radiance(LumRadContext ctx, float* rgb) {
     Context* c = as_ctx(ctx);
     if (!c || !rgb) return fail(LUMRAD_EINVAL, "null argument");
     LUMRAD_TRY(cudaSetDevice(c->device));
     DeviceWorld& w = c->world;
     const size_t bytes = w.W * 3 * sizeof(float);
-    // packed to RGB floats on the device (FP16/BF16 widened exactly); one copy, straight into the
-    // caller's array when it is page-locked, else through the context's pinned buffer
-    const bool direct = host_pinned(rgb, bytes);
-    if (!c->d_rgb) LUMRAD_TRY(cudaMalloc(&c->d_rgb, bytes));
-    if (!direct && !c->h_rgb) LUMRAD_TRY(cudaMallocHost(&c->h_rgb, bytes));
-    LUMRAD_TRY(launch_pack_rgb(w.d_rad[w.cur], w.precision, (long long)w.W, c->d_rgb, c->stream));
-    LUMRAD_TRY(cudaMemcpyAsync(direct ? rgb : c->h_rgb, c->d_rgb, bytes, cudaMemcpyDeviceToHost, c->stream));
-    LUMRAD_TRY(cudaMemcpyAsync(c->h_err, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    // packed to RGB floats by the device (FP16/BF16 widened exactly) straight into the caller's array
+    // when it is page-locked, else into the context's page-locked buffer
+    float* out = static_cast<float*>(pinned_device_range(rgb, bytes));
+    const bool direct = out != nullptr;
+    if (!direct) {
+        if (!c->h_rgb) LUMRAD_TRY(cudaMallocHost(&c->h_rgb, bytes));
+        LUMRAD_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&out), c->h_rgb, 0));
+    }
+    int* err_out = nullptr;
+    LUMRAD_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&err_out), c->h_err, 0));
+    LUMRAD_TRY(launch_pack_rgb(w.d_rad[w.cur], w.precision, (long long)w.W, out, c->d_error, err_out, c->stream));
     LUMRAD_TRY(cudaStreamSynchronize(c->stream));   // one wait for the volume and the error word
     if (!direct) std::memcpy(rgb, c->h_rgb, bytes);
     return c->have_pass ? c->handle_error(*c->h_err) : LUMRAD_OK;

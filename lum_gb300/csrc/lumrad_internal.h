@@ -228,8 +228,10 @@ cudaError_t launch_shift_radiance(const void* src, void* dst, int X, int Y, int 
 cudaError_t launch_gather(const void* rad, int X, int Y, int Z, int precision, const float* pts, int n, float* out,
                           cudaStream_t stream);
 
-// The volume rad (W probes, storage `precision`) as W*3 packed floats.
-cudaError_t launch_pack_rgb(const void* rad, int precision, long long W, float* out, cudaStream_t stream);
+// The volume rad (W probes, storage `precision`) as W*3 packed floats at `out`, and *err at `err_out`
+// (device addresses of page-locked host memory, or device memory).
+cudaError_t launch_pack_rgb(const void* rad, int precision, long long W, float* out, const int* err, int* err_out,
+                            cudaStream_t stream);
 
 // One mesh of map.comp: column-major inverse transform (float), the dispatch origin in world
 // voxels (pco.shift) and the dispatch size in voxels (a multiple of 4 per axis).

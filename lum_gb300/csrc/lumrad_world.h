@@ -213,8 +213,7 @@ struct Context {
     uint8_t* d_dirty_mask = nullptr;      // 2 W bytes: the dirty-probe dilation's ping-pong masks
     short4* d_edits = nullptr;
     size_t edits_cap = 0;
-    // volume read-back: packed RGB on the device, pinned staging on the host
-    float* d_rgb = nullptr;
+    // volume read-back into arrays that are not page-locked: the page-locked buffer the device writes
     float* h_rgb = nullptr;
     // gather staging (host-buffer calls)
     float* d_gather = nullptr;
