@@ -137,7 +137,7 @@ class RadianceWorld:
         """Probes within `radius` blocks of the edits, derived on the device; (n, 4) int16."""
         e = _edits(edits)
         n = C.c_int()
-        out = np.zeros((self.n_blocks, 4), dtype=np.int16)
+        out = np.empty((self.n_blocks, 4), dtype=np.int16)
         check(self.lib.lumrad_build_dirty_list(self.h, e.ctypes.data if e.size else None, e.size, radius, ptr(out),
                                                self.n_blocks, C.byref(n)))
         return out[: n.value]

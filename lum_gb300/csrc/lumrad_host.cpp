@@ -667,7 +667,22 @@ int Context::ensure_list_scratch() {
         LUMRAD_TRY(cudaMalloc(&list.listed, sizeof(int)));
         LUMRAD_TRY(cudaMalloc(&d_list_count, sizeof(int)));
         LUMRAD_TRY(cudaMallocHost(&h_list_count, sizeof(int)));
+        LUMRAD_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&h_list_count_dev), h_list_count, 0));
     }
+    return LUMRAD_OK;
+}
+
+// Page-locked room for a list of every block and, after it, n edits.
+int Context::ensure_list_staging(size_t n) {
+    if (world.W + n <= h_list_cap) return LUMRAD_OK;
+    LUMRAD_TRY(cudaStreamSynchronize(stream));
+    if (h_list) cudaFreeHost(h_list);
+    h_list = nullptr;
+    h_list_cap = 0;
+    const size_t cap = world.W + std::max<size_t>(2 * n, 1024);
+    LUMRAD_TRY(cudaMallocHost(&h_list, cap * sizeof(short4)));
+    LUMRAD_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&h_list_dev), h_list, 0));
+    h_list_cap = cap;
     return LUMRAD_OK;
 }
 
@@ -734,6 +749,7 @@ void Context::release() {
     cudaFree(d_specials);
     cudaFree(d_list_count);
     if (h_list_count) cudaFreeHost(h_list_count);
+    if (h_list) cudaFreeHost(h_list);
     cudaFree(d_dirty_mask);
     cudaFree(d_edits);
     cudaFree(d_gather);
@@ -1062,6 +1078,17 @@ int lumrad_build_dirty_list(LumRadContext ctx, const LumRadEdit* edits, int n_ed
     LUMRAD_TRY(cudaSetDevice(c->device));
     int rc = c->ensure_list_scratch();
     if (rc) return rc;
+    if (dirty_rows_fit((long long)w.W, n_edits, radius)) {
+        // edits read from, list and length written to page-locked memory: no copies, one wait
+        if ((rc = c->ensure_list_staging((size_t)n_edits))) return rc;
+        if (n_edits > 0) std::memcpy(c->h_list + w.W, edits, (size_t)n_edits * sizeof(short4));
+        LUMRAD_TRY(launch_dirty_rows(c->h_list_dev + w.W, n_edits, w.X, w.Y, w.Z, radius, c->list.bits, c->h_list_dev,
+                                     c->h_list_count_dev, c->stream));
+        LUMRAD_TRY(cudaStreamSynchronize(c->stream));
+        *n = *c->h_list_count;
+        if (cap > 0 && *n > 0) std::memcpy(out, c->h_list, (size_t)std::min(*n, cap) * sizeof(short4));
+        return LUMRAD_OK;
+    }
     if ((rc = c->ensure_req_capacity(w.W))) return rc;
     if (!c->d_dirty_mask) LUMRAD_TRY(cudaMalloc(&c->d_dirty_mask, 2 * w.W));
     if ((size_t)n_edits > c->edits_cap) {

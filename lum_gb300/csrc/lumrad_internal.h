@@ -194,7 +194,7 @@ cudaError_t launch_passes(const LaunchArgs& args, const WorldPass* h_tab, int n_
 cudaError_t launch_prep(const WorldPass* d_worlds, int n_worlds, int precision, cudaStream_t stream,
                         const int* dev_n = nullptr);
 
-// Device scratch of the update-list builder for a world of W blocks: ceil(W/32) flag words,
+// Device scratch of the update-list builder for a world of W blocks: 8 * ceil(W/256) flag words,
 // ceil(W/256) CTA counts and offsets, and the count of rule-listed blocks.
 struct ListScratch {
     uint32_t* bits;
@@ -217,6 +217,12 @@ cudaError_t launch_update_list(const int16_t* grid, int X, int Y, int Z, const s
 cudaError_t launch_dirty_list(const short4* edits, int n_edits, int X, int Y, int Z, int radius, uint8_t* mask_a,
                               uint8_t* mask_b, const ListScratch& scratch, short4* out, int* count,
                               cudaStream_t stream);
+
+// The same for a few edits (dirty_rows_fit), without masks: bits are the list scratch's; edits and out
+// may be page-locked host memory's device addresses.
+bool dirty_rows_fit(long long W, int n_edits, int radius);
+cudaError_t launch_dirty_rows(const short4* edits, int n_edits, int X, int Y, int Z, int radius, uint32_t* bits, short4* out,
+                              int* count, cudaStream_t stream);
 
 // shift_radiance (internal_render.cpp:1218-1335) from src into dst: dst(p) = src(p + shift)
 // where p + shift is inside the world, src(p) elsewhere.

@@ -210,6 +210,11 @@ struct Context {
     size_t specials_cap = 0;
     int* d_list_count = nullptr;
     int* h_list_count = nullptr;          // pinned
+    int* h_list_count_dev = nullptr;      // its device address
+    // page-locked list staging of build_dirty_list (W entries, then the call's edits)
+    short4* h_list = nullptr;
+    short4* h_list_dev = nullptr;
+    size_t h_list_cap = 0;
     uint8_t* d_dirty_mask = nullptr;      // 2 W bytes: the dirty-probe dilation's ping-pong masks
     short4* d_edits = nullptr;
     size_t edits_cap = 0;
@@ -243,6 +248,7 @@ struct Context {
     // is set.
     int build_list_device(bool consume, int* n);
     int ensure_list_scratch();
+    int ensure_list_staging(size_t n);
     int shift_volume(int dx, int dy, int dz);
     void release();
 };

@@ -116,10 +116,10 @@ list_scan_kernel(const int* __restrict__ counts, int n, int* __restrict__ offset
     if (threadIdx.x == 0) *total = carry;
 }
 
-// The list from the bits.  A CTA's offset: offsets[blockIdx.x] of a scan of the counts, or, with
-// offsets null (up to kDirectCtas CTAs), the sum of the counts before its own, formed here; the last
-// CTA then also writes the length.
-constexpr int kDirectCtas = 4096;
+// The list from the bits.  A CTA's offset: offsets[blockIdx.x] of a scan of the counts; or, offsets
+// null (up to kDirectCtas CTAs), the sum of the counts before its own; or, both null (up to
+// kBitsCtas), of the bits before its own; the last CTA then also writes the length.
+constexpr int kDirectCtas = 4096, kBitsCtas = 1024;
 __global__ void __launch_bounds__(kListCta)
 list_write_kernel(const uint32_t* __restrict__ bits, const int* __restrict__ counts, const int* __restrict__ offsets, int X,
                   int Y, unsigned W, short4* __restrict__ out, int* __restrict__ total, int* __restrict__ total2) {
@@ -131,7 +131,13 @@ list_write_kernel(const uint32_t* __restrict__ bits, const int* __restrict__ cou
     grid_dependency_wait();
     const uint32_t b = i < W ? __ldcg(bits + (i >> 5)) : 0u;
     int sum = 0;
-    if (!offsets)
+    if (!counts) {   // (a CTA's words: two uint4)
+        const uint4* v = reinterpret_cast<const uint4*>(bits);
+        for (int c = threadIdx.x; c < 2 * (int)blockIdx.x; c += kListCta) {
+            const uint4 x = __ldcg(v + c);
+            sum += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+        }
+    } else if (!offsets)
         for (int c = threadIdx.x; c < (int)blockIdx.x; c += kListCta) sum += __ldcg(counts + c);
     sum = __reduce_add_sync(kFull, sum);
     if (lane == 0) {
@@ -166,6 +172,30 @@ cudaError_t launch_list_write(const ListScratch& s, int X, int Y, long long W, s
     }
     return launch_kernel(list_write_kernel, ctas, kListCta, 0, stream, false, s.bits, s.cta_counts, s.cta_offsets, X, Y,
                          (unsigned)W, out, nullptr, nullptr);
+}
+
+// Dirty probes of a few edits (Chebyshev distance <= r): each row of an edit's cube sets its run of
+// bits, a thread per row; the list is then written from the bits.  A memset and two launches,
+// where the dilation below takes a memset and five: used while the rows are at most 2^21 and the
+// world at most 262,144 blocks.
+__global__ void dirty_rows_kernel(const short4* __restrict__ edits, int rows, int X, int Y, int Z, int r,
+                                  uint32_t* __restrict__ bits) {
+    grid_launch_dependents();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= rows) return;
+    const int side = 2 * r + 1, row = k % (side * side);
+    const short4 e = edits[k / (side * side)];
+    const int y = e.y + row % side - r, z = e.z + row / side - r;
+    if (y < 0 || y >= Y || z < 0 || z >= Z) return;
+    const int x0 = max(e.x - r, 0), x1 = min(e.x + r, X - 1);   // at most 31 blocks: two words
+    const unsigned i0 = (unsigned)x0 + (unsigned)X * ((unsigned)y + (unsigned)Y * (unsigned)z), i1 = i0 + (unsigned)(x1 - x0);
+    const uint32_t m0 = ~0u << (i0 & 31), m1 = ~0u >> (31 - (i1 & 31));
+    if ((i0 >> 5) == (i1 >> 5)) {
+        atomicOr(bits + (i0 >> 5), m0 & m1);
+    } else {
+        atomicOr(bits + (i0 >> 5), m0);
+        atomicOr(bits + (i1 >> 5), m1);
+    }
 }
 
 // Dirty probes of block edits (Chebyshev distance <= r): a byte mask of the edited blocks, dilated
@@ -614,7 +644,24 @@ cudaError_t launch_dirty_list(const short4* edits, int n_edits, int X, int Y, in
     return launch_list_write(s, X, Y, W, out, count, nullptr, stream);
 }
 
-size_t list_scratch_words(long long W) { return (size_t)((W + 31) / 32); }
+bool dirty_rows_fit(long long W, int n_edits, int radius) {
+    const long long side = 2LL * radius + 1;
+    return list_scratch_ctas(W) <= kBitsCtas && n_edits * side * side <= 1LL << 21;
+}
+
+cudaError_t launch_dirty_rows(const short4* edits, int n_edits, int X, int Y, int Z, int radius, uint32_t* bits, short4* out,
+                              int* count, cudaStream_t stream) {
+    const long long W = (long long)X * Y * Z;
+    const long long rows = (long long)n_edits * (2 * radius + 1) * (2 * radius + 1);
+    cudaError_t e = cudaMemsetAsync(bits, 0, list_scratch_words(W) * sizeof(uint32_t), stream);
+    if (e != cudaSuccess) return e;
+    if (rows > 0) dirty_rows_kernel<<<(int)((rows + 255) / 256), 256, 0, stream>>>(edits, (int)rows, X, Y, Z, radius, bits);
+    return launch_kernel(list_write_kernel, (int)list_scratch_ctas(W), kListCta, 0, stream, true, bits, nullptr, nullptr, X, Y,
+                         (unsigned)W, out, count, nullptr);
+}
+
+// (whole CTAs' words: the list's writer reads its own and those before them)
+size_t list_scratch_words(long long W) { return (size_t)((W + kListCta - 1) / kListCta) * (kListCta / 32); }
 size_t list_scratch_ctas(long long W) { return (size_t)((W + kListCta - 1) / kListCta); }
 
 cudaError_t launch_shift_radiance(const void* src, void* dst, int X, int Y, int Z, int sx, int sy, int sz,

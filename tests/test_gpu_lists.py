@@ -67,3 +67,19 @@ def test_frames_back_to_back(dims):
             b.radiance_pass(req, p[k])
             assert b.gather(pts).tobytes() == outs[k].cpu().numpy().tobytes()
         assert a.get_radiance().tobytes() == b.get_radiance().tobytes()
+
+
+@pytest.mark.parametrize("dims", [(31, 9, 5), (64, 64, 64), (2047, 3, 2), (65, 64, 64)])
+@pytest.mark.parametrize("n,radius", [(0, 2), (1, 0), (1, 15), (700, 3), (2200, 15)])
+def test_dirty_lists(dims, n, radius):
+    """Both forms of the dirty list (rows of bits; the dilation of larger worlds and edit counts)."""
+    import lum_gb300
+    rng = np.random.default_rng(n + radius)
+    edits = np.zeros((n, 4), np.int16)
+    for a in range(3):
+        edits[:, a] = rng.choice([0, dims[a] - 1, dims[a] // 2, -1], n) if n else 0
+        wild = edits[:, a] < 0
+        edits[wild, a] = rng.integers(0, dims[a], int(wild.sum()))
+    with lum_gb300.RadianceWorld(dims, max_block_types=4) as rw:
+        for _ in range(2):
+            assert np.array_equal(rw.build_dirty_list(edits, radius), lum_gb300.dirty_probes(dims, edits, radius))
