@@ -82,6 +82,7 @@ int build(Batch* b) {
         BatchWorld& bw = b->worlds[i];
         if (!bw.set) return fail(LUMRAD_ESTATE, "every world of a batch needs lumrad_batch_set_requests");
         WorldPass w;
+        if (!bw.ctx->world.edited.empty()) bw.ctx->world.grid_dirty = true;   // uploaded and waited for
         if ((rc = bw.ctx->world.fill_pass(bw.d_req, bw.n, bw.p, b->stream, &w))) return rc;
         w.task_begin = begin;
         begin += (w.n_tasks + kWarps - 1) / kWarps * kWarps;

@@ -114,20 +114,34 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
     int rc = w.sync_inputs(c->stream);   // the origin world and palette as loaded
     if (rc) return rc;
 
-    // page-locked staging (see Context::h_blk), made on the first call
-    const size_t off_cgrid = w.W * sizeof(int16_t), off_cslot = off_cgrid + (compact_cells(w.X, w.Y, w.Z) * sizeof(uint16_t) + 15) / 16 * 16;
-    const size_t n_cslot = (size_t)w.n_slots + 128;
-    const size_t off_copies = off_cslot + n_cslot * sizeof(int);
-    if (!c->h_blk) {
-        LUMRAD_TRY(cudaMallocHost(&c->h_blk, off_copies + (size_t)w.n_slots * sizeof(int2)));
-        LUMRAD_TRY(cudaMalloc(&c->d_blk_copies, (size_t)w.n_slots * sizeof(int2)));
+    // this half of the staging (see Context::h_blk), made on its first use
+    const int half = c->blk_half;
+    if (!c->h_blk[half]) {
+        LUMRAD_TRY(cudaMallocHost(&c->h_blk[half], (size_t)w.n_slots * sizeof(int2)));
+        LUMRAD_TRY(cudaEventCreateWithFlags(&c->ev_blk[half], cudaEventDisableTiming));
+    } else {
+        LUMRAD_TRY(cudaEventSynchronize(c->ev_blk[half]));
     }
-    int16_t* cur = reinterpret_cast<int16_t*>(c->h_blk);   // the previous call's uploads are done
-    int2* copies = reinterpret_cast<int2*>(c->h_blk + off_copies);
-    std::memcpy(cur, w.h_grid.data(), w.W * sizeof(int16_t));
+    int2* copies = c->h_blk[half];
     int n_copies = 0;
 
-    // blockify (host): temporary slots from static_blocks up, in mesh order
+    // blockify (host): temporary slots from static_blocks up, in mesh order, over the origin world:
+    // the last frame's blocks get their origin ids again, this frame's are listed
+    if (w.h_cur.empty()) w.h_cur = w.h_grid;
+    int16_t* cur = w.h_cur.data();
+    std::vector<std::pair<uint32_t, int16_t>> last;   // the last frame's ids, put back if this one fails
+    std::vector<uint32_t> cells = w.blk_cells;        // the last frame's blocks, then this one's
+    last.reserve(cells.size());
+    for (uint32_t i : cells) {
+        last.emplace_back(i, cur[i]);
+        cur[i] = w.h_grid[i];
+    }
+    const size_t first_new = cells.size();
+    auto undo = [&](int code) {
+        for (size_t k = first_new; k < cells.size(); k++) cur[cells[k]] = w.h_grid[cells[k]];
+        for (const auto& e : last) cur[e.first] = e.second;
+        return code;
+    };
     int counter = static_blocks;
     for (int i = 0; i < n_meshes; i++) {
         float r[3][3];
@@ -144,19 +158,21 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
         for (int z = lo[2]; z <= hi[2]; z++)
             for (int y = lo[1]; y <= hi[1]; y++)
                 for (int x = lo[0]; x <= hi[0]; x++) {
-                    int16_t& b = cur[(size_t)x + (size_t)w.X * ((size_t)y + (size_t)w.Y * z)];
+                    const size_t at = (size_t)x + (size_t)w.X * ((size_t)y + (size_t)w.Y * z);
+                    int16_t& b = cur[at];
                     if (b >= static_blocks) continue;   // already temporary (or a dynamic id): left as is
                     if (counter >= w.n_slots || counter > 32767)
-                        return fail(LUMRAD_ENOMEM, "temporary blocks exceed max_block_types");
+                        return undo(fail(LUMRAD_ENOMEM, "temporary blocks exceed max_block_types"));
                     // copy the static block's voxels; a negative id has no source block (the
                     // reference's copy would start at a negative palette offset)
                     if (b > 0) copies[n_copies++] = make_int2(b, counter);
                     b = (int16_t)counter++;
+                    cells.push_back((uint32_t)at);
                 }
     }
 
     // map dispatches of every mesh (checked before anything reaches the device)
-    std::vector<MapArgs> margs(n_meshes);
+    std::vector<MapMesh> mesh(n_meshes);
     for (int i = 0; i < n_meshes; i++) {
         float r[3][3];
         quat_to_mat(transforms[i].rot, r);
@@ -164,16 +180,18 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
         const Context::Model& m = c->models[models[i]];
         const int size[3] = {m.sx, m.sy, m.sz};
         const Box box = model_aabb(r, s, size);
-        MapArgs& a = margs[i];
+        mesh[i].voxels = m.d_vox;
+        MapArgs& a = mesh[i].a;
         double invocations = 1.0;
         for (int k = 0; k < 3; k++) {
+            mesh[i].size[k] = size[k];
             const int mn = (int)std::floor(box.mn[k]);   // ivec3(floor(min)), ivec3(ceil(max)) (:1500-1501)
             const int mx = (int)std::ceil(box.mx[k]);
             a.shift[k] = mn;
             a.dims[k] = (mx - mn + 3) / 4 * 4;   // (map_area + 3) / 4 groups of 4 (:1512)
             invocations *= (double)a.dims[k];
         }
-        if (invocations >= 4294967296.0) return fail(LUMRAD_EINVAL, "a mesh covers more than 2^32 world voxels");
+        if (invocations >= 4294967296.0) return undo(fail(LUMRAD_EINVAL, "a mesh covers more than 2^32 world voxels"));
         // inverse [R^T | -R^T s], column-major
         for (int col = 0; col < 3; col++)
             for (int row = 0; row < 3; row++) a.inv[4 * col + row] = r[row][col];
@@ -187,25 +205,40 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
 
     // the slots this frame writes: every id from static_blocks up present in the grid (made here
     // or set by the caller), below n_slots
-    int used_end = static_blocks;
-    for (size_t i = 0; i < w.W; i++) used_end = std::max(used_end, (int)cur[i] + 1);
-    used_end = std::min(used_end, w.n_slots);
+    if (w.origin_end < 0) {
+        w.origin_end = 0;
+        for (size_t i = 0; i < w.W; i++) w.origin_end = std::max(w.origin_end, (int)w.h_grid[i] + 1);
+    }
+    const int used_end = std::min(std::max(std::max(counter, w.origin_end), static_blocks), w.n_slots);
+    // the changed blocks into the device's grids; if an id needs a wider compact grid, the whole world
+    bool fits = true;
+    if ((rc = w.apply_cells(cells.data(), cells.size(), cur, false, c->stream, &fits))) return undo(rc);
+    if (!fits) {
+        w.uploads++;
+        w.build_compact(cur, false);   // the occupancy masks come from the device palette below
+        if ((rc = w.ensure_compact_room(c->stream))) return undo(rc);
+        LUMRAD_TRY(cudaMemcpyAsync(w.d_grid, cur, w.W * sizeof(int16_t), cudaMemcpyHostToDevice, c->stream));
+        LUMRAD_TRY(cudaMemcpyAsync(w.d_cgrid, w.h_cgrid.data(), w.h_cgrid.size(), cudaMemcpyHostToDevice, c->stream));
+        LUMRAD_TRY(cudaMemcpyAsync(w.d_cslot, w.h_cslot.data(), w.h_cslot.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+        LUMRAD_TRY(cudaStreamSynchronize(c->stream));   // host vectors may be rebuilt by the next call
+    }
+    w.blk_cells.assign(cells.begin() + (std::ptrdiff_t)first_new, cells.end());
     // exec_copies (device): temporary part of the palette cleared (the slots that may hold voxels:
-    // the rest are zero already), block copies, world upload
+    // the rest are zero already), block copies
     const int clear_end = std::min(std::max(used_end, w.pal_dirty_end), w.n_slots);
     if (clear_end > static_blocks)
         LUMRAD_TRY(cudaMemsetAsync(w.d_pal + (size_t)static_blocks * 4096, 0, (size_t)(clear_end - static_blocks) * 4096,
                                    c->stream));
     w.pal_dirty_end = used_end;
+    w.uploads++;
     if (n_copies > 0) {
-        LUMRAD_TRY(cudaMemcpyAsync(c->d_blk_copies, copies, (size_t)n_copies * sizeof(int2), cudaMemcpyHostToDevice,
-                                   c->stream));
-        LUMRAD_TRY(launch_palette_copies(w.d_pal, c->d_blk_copies, n_copies, c->stream));
+        int2* dev = nullptr;
+        LUMRAD_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev), copies, 0));
+        LUMRAD_TRY(launch_palette_copies(w.d_pal, dev, n_copies, c->stream));
     }
-    LUMRAD_TRY(cudaMemcpyAsync(w.d_grid, cur, w.W * sizeof(int16_t), cudaMemcpyHostToDevice, c->stream));
 
-    // map (device), mesh by mesh; writes claimed in the owner words (one per voxel of the slots
-    // in use: the map writes only into blocks of the grid), then resolved
+    // map (device); writes claimed in the owner words (one per voxel of the slots in use: the map
+    // writes only into blocks of the grid), then resolved
     const size_t n_tmp = (size_t)(used_end - static_blocks) * 4096;
     if (n_meshes > 0 && n_tmp > 0) {
         if (n_tmp > c->map_owner_cap) {
@@ -217,42 +250,14 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
             c->map_owner_cap = n_tmp;
         }
         LUMRAD_TRY(cudaMemsetAsync(c->d_map_owner, 0, n_tmp * sizeof(unsigned long long), c->stream));
-    }
-    for (int i = 0; i < n_meshes && n_tmp > 0; i++) {
-        const Context::Model& m = c->models[models[i]];
-        LUMRAD_TRY(launch_map(w.d_grid, w.X, w.Y, w.Z, w.n_slots, static_blocks, m.d_vox, m.sx, m.sy, m.sz, margs[i], i,
-                              c->d_map_owner, c->stream));
-    }
-    if (n_meshes > 0 && n_tmp > 0)
+        LUMRAD_TRY(launch_map(w.d_grid, w.X, w.Y, w.Z, w.n_slots, static_blocks, mesh.data(), n_meshes, 0, c->d_map_owner,
+                              c->stream));
         LUMRAD_TRY(launch_map_resolve(w.d_pal + (size_t)static_blocks * 4096, c->d_map_owner, n_tmp, c->stream));
-
-    // compact world of the blockified grid; occupancy masks from the device palette
-    w.build_compact(cur, false);   // the occupancy masks come from the device palette below
-    const size_t cap = std::max<size_t>((size_t)w.n_compact, (size_t)w.n_slots + 64);
-    if (cap > w.cbits_cap) {
-        LUMRAD_TRY(cudaStreamSynchronize(c->stream));
-        cudaFree(w.d_cbits);
-        cudaFree(w.d_cslot);
-        w.d_cbits = nullptr;
-        w.d_cslot = nullptr;
-        w.cbits_cap = 0;
-        LUMRAD_TRY(cudaMalloc(&w.d_cbits, cap * 128 * sizeof(uint32_t)));
-        LUMRAD_TRY(cudaMalloc(&w.d_cslot, cap * sizeof(int)));
-        w.cbits_cap = cap;
     }
-    // the compact grid and slots through the staging area (both fit: uint16 ids at most, and
-    // at most n_slots + 66 compact ids)
-    const void* cslot_src = w.h_cslot.data();
-    if (w.h_cslot.size() <= n_cslot) {
-        std::memcpy(c->h_blk + off_cslot, w.h_cslot.data(), w.h_cslot.size() * sizeof(int));
-        cslot_src = c->h_blk + off_cslot;
-    }
-    std::memcpy(c->h_blk + off_cgrid, w.h_cgrid.data(), w.h_cgrid.size());
-    LUMRAD_TRY(cudaMemcpyAsync(w.d_cslot, cslot_src, w.h_cslot.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    // the occupancy masks from the device palette
     LUMRAD_TRY(launch_compact_bits(w.d_pal, w.d_cslot, w.n_compact, w.d_cbits, c->stream));
-    LUMRAD_TRY(cudaMemcpyAsync(w.d_cgrid, c->h_blk + off_cgrid, w.h_cgrid.size(), cudaMemcpyHostToDevice, c->stream));
-    w.h_cur.assign(cur, cur + w.W);
-    LUMRAD_TRY(cudaStreamSynchronize(c->stream));   // the staging area is reused by the next call
+    LUMRAD_TRY(cudaEventRecord(c->ev_blk[half], c->stream));
+    c->blk_half ^= 1;
     return LUMRAD_OK;
 }
 

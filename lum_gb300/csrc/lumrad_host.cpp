@@ -89,6 +89,13 @@ void DeviceWorld::release() {
     cudaFree(d_grid); cudaFree(d_cgrid); cudaFree(d_cbits); cudaFree(d_cslot); cudaFree(d_pal); cudaFree(d_mats);
     cudaFree(d_rad[0]); cudaFree(d_rad[1]); cudaFree(d_scratch); cudaFree(d_probe_count); cudaFree(d_stats);
     cudaFree(d_hits);
+    for (int h = 0; h < 2; h++) {
+        if (h_cells[h]) cudaFreeHost(h_cells[h]);
+        if (ev_cells[h]) cudaEventDestroy(ev_cells[h]);
+        h_cells[h] = nullptr;
+        ev_cells[h] = nullptr;
+        cells_cap[h] = 0;
+    }
     for (auto& kv : d_dirs) cudaFree(kv.second);
     d_dirs.clear();
     d_grid = nullptr; d_cgrid = nullptr; d_cbits = nullptr; d_cslot = nullptr; d_pal = nullptr; d_mats = nullptr;
@@ -201,33 +208,91 @@ size_t DeviceWorld::footprint() const {
     return b;
 }
 
+int DeviceWorld::ensure_compact_room(cudaStream_t stream) {
+    // room for every id that has a palette slot (-63..-1, 1..n_slots-1), air and the empty id, so ids
+    // that edits bring in later never reallocate
+    const size_t cap = std::max<size_t>((size_t)n_compact, (size_t)n_slots + 64);
+    if (cap <= cbits_cap) return LUMRAD_OK;
+    LUMRAD_TRY(cudaStreamSynchronize(stream));
+    cudaFree(d_cbits);
+    cudaFree(d_cslot);
+    d_cbits = nullptr;
+    d_cslot = nullptr;
+    cbits_cap = 0;
+    LUMRAD_TRY(cudaMalloc(&d_cbits, cap * 128 * sizeof(uint32_t)));
+    LUMRAD_TRY(cudaMalloc(&d_cslot, cap * sizeof(int)));
+    cbits_cap = cap;
+    return LUMRAD_OK;
+}
+
+int DeviceWorld::apply_cells(const uint32_t* idx, size_t n, const int16_t* g, bool host_bits, cudaStream_t stream, bool* fits) {
+    *fits = true;
+    if (n == 0) return LUMRAD_OK;
+    const int h = cells_half;
+    if (ev_cells[h]) LUMRAD_TRY(cudaEventSynchronize(ev_cells[h]));   // this half's last kernel has read it
+    else LUMRAD_TRY(cudaEventCreateWithFlags(&ev_cells[h], cudaEventDisableTiming));
+    if (n > cells_cap[h]) {
+        if (h_cells[h]) cudaFreeHost(h_cells[h]);
+        h_cells[h] = nullptr;
+        cells_cap[h] = 0;
+        const size_t cap = std::max<size_t>(2 * n, 1024);
+        LUMRAD_TRY(cudaMallocHost(&h_cells[h], cap * sizeof(CellEdit)));
+        cells_cap[h] = cap;
+    }
+    const int first_new = n_compact;
+    skip_host_bits = !host_bits;
+    for (size_t k = 0; k < n && *fits; k++) {
+        bool assigned = false;
+        const int16_t b = g[idx[k]];
+        const int c = compact_of(b, &assigned);
+        if (c < 0) *fits = false;
+        h_cells[h][k] = CellEdit{idx[k], b, (uint16_t)c};
+    }
+    skip_host_bits = false;
+    if (!*fits) return LUMRAD_OK;   // (the caller rebuilds the compact world)
+    uploads++;
+    if ((size_t)n_compact > cbits_cap) return fail(LUMRAD_EDEVICE, "compact ids past their reserved room");   // cannot happen
+    if (n_compact > first_new) {    // (pageable copies: staged before the call returns)
+        const size_t m = (size_t)(n_compact - first_new);
+        if (host_bits)
+            LUMRAD_TRY(cudaMemcpyAsync(d_cbits + (size_t)first_new * 128, h_cbits.data() + (size_t)first_new * 128,
+                                       m * 128 * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
+        LUMRAD_TRY(cudaMemcpyAsync(d_cslot + first_new, h_cslot.data() + first_new, m * sizeof(int), cudaMemcpyHostToDevice, stream));
+    }
+    CellEdit* dev = nullptr;
+    LUMRAD_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev), h_cells[h], 0));
+    LUMRAD_TRY(launch_apply_cells(dev, (int)n, d_grid, d_cgrid, cgrid_wide, X, Y, stream));
+    LUMRAD_TRY(cudaEventRecord(ev_cells[h], stream));
+    cells_half ^= 1;
+    return LUMRAD_OK;
+}
+
 int DeviceWorld::sync_inputs(cudaStream_t stream) {
+    if (!grid_dirty && !compact_dirty && !edited.empty()) {
+        bool fits = true;
+        const int rc = apply_cells(edited.data(), edited.size(), h_grid.data(), true, stream, &fits);
+        if (rc) return rc;
+        edited.clear();
+        if (fits) return LUMRAD_OK;
+        grid_dirty = true;   // more than 256 ids: the whole world again, with uint16 compact ids
+    }
+    edited.clear();
     // a changed origin world or palette replaces the blockified frame (the next blockify rebuilds it)
     if (!h_cur.empty() && (grid_dirty || compact_dirty)) {
         h_cur.clear();
+        blk_cells.clear();
         grid_dirty = true;
     }
     if (grid_dirty || compact_dirty) uploads++;
     if (grid_dirty) {
+        origin_end = -1;
         LUMRAD_TRY(cudaMemcpyAsync(d_grid, h_grid.data(), W * sizeof(int16_t), cudaMemcpyHostToDevice, stream));
         grid_dirty = false;
         compact_dirty = true;
     }
     if (compact_dirty) {
         build_compact();
-        // room for every id that has a palette slot (-63..-1, 1..n_slots-1), air and the empty id,
-        // so ids that edits bring in later never reallocate
-        const size_t cap = std::max<size_t>((size_t)n_compact, (size_t)n_slots + 64);
-        if (cap > cbits_cap) {
-            cudaFree(d_cbits);
-            cudaFree(d_cslot);
-            d_cbits = nullptr;
-            d_cslot = nullptr;
-            cbits_cap = 0;
-            LUMRAD_TRY(cudaMalloc(&d_cbits, cap * 128 * sizeof(uint32_t)));
-            LUMRAD_TRY(cudaMalloc(&d_cslot, cap * sizeof(int)));
-            cbits_cap = cap;
-        }
+        if (int rc = ensure_compact_room(stream)) return rc;
         LUMRAD_TRY(cudaMemcpyAsync(d_cgrid, h_cgrid.data(), h_cgrid.size(), cudaMemcpyHostToDevice, stream));
         LUMRAD_TRY(cudaMemcpyAsync(d_cbits, h_cbits.data(), h_cbits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
                                    stream));
@@ -690,6 +755,10 @@ int Context::build_list_device(bool consume, int* n) {
     NvtxRange range("lumrad update list");
     int rc = world.sync_inputs(stream);
     if (rc) return rc;
+    // (the list's first launch reads the grid while the kernel before it may still run: not after one
+    // that writes the grid)
+    const bool dependent = world.uploads == list_uploads;
+    list_uploads = world.uploads;
     const long long W = (long long)world.W;
     if ((rc = ensure_list_scratch())) return rc;
     const size_t ns = specials.size() / 4;
@@ -704,7 +773,7 @@ int Context::build_list_device(bool consume, int* n) {
     }
     if (ns) LUMRAD_TRY(cudaMemcpyAsync(d_specials, specials.data(), ns * sizeof(short4), cudaMemcpyHostToDevice, stream));
     LUMRAD_TRY(launch_update_list(world.d_grid, world.X, world.Y, world.Z, d_specials, (int)ns, list, d_req,
-                                  d_list_count, stream));
+                                  d_list_count, dependent, stream));
     if (consume) specials.clear();
     if (!n) return LUMRAD_OK;   // the length stays on the device
     LUMRAD_TRY(cudaMemcpyAsync(h_list_count, d_list_count, sizeof(int), cudaMemcpyDeviceToHost, stream));
@@ -757,11 +826,13 @@ void Context::release() {
     for (auto& m : models) cudaFree(m.d_vox);
     models.clear();
     cudaFree(d_map_owner);
-    if (h_blk) cudaFreeHost(h_blk);
+    for (int h = 0; h < 2; h++) {
+        if (h_blk[h]) cudaFreeHost(h_blk[h]);
+        if (ev_blk[h]) cudaEventDestroy(ev_blk[h]);
+    }
     cudaFree(d_last_count);
     cudaFree(d_pass_mask);
     cudaFree(d_pass_mask2);
-    cudaFree(d_blk_copies);
     if (h_err) cudaFreeHost(h_err);
     if (ev_req) cudaEventDestroy(ev_req);
     cudaFree(d_ptime);
@@ -879,8 +950,13 @@ int lumrad_set_world_block(LumRadContext ctx, int x, int y, int z, int16_t block
     DeviceWorld& w = c->world;
     if (x < 0 || y < 0 || z < 0 || x >= w.X || y >= w.Y || z >= w.Z)
         return fail(LUMRAD_EINVAL, "block coordinate out of the world");
-    w.h_grid[(size_t)x + (size_t)w.X * ((size_t)y + (size_t)w.Y * z)] = block;
-    w.grid_dirty = true;   // uploaded before the next pass, as exec_copies does every frame
+    const size_t idx = (size_t)x + (size_t)w.X * ((size_t)y + (size_t)w.Y * z);
+    w.h_grid[idx] = block;
+    if (w.origin_end >= 0) w.origin_end = std::max(w.origin_end, (int)block + 1);
+    // uploaded before the next pass, as exec_copies does every frame: block by block while they are
+    // few (an eighth of the world) and no blockified frame has to give way to the changed world
+    if (!w.grid_dirty && !w.compact_dirty && w.h_cur.empty() && w.edited.size() < w.W / 8 + 64) w.edited.push_back((uint32_t)idx);
+    else w.grid_dirty = true;
     return LUMRAD_OK;
 }
 

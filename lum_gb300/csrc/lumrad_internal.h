@@ -208,8 +208,9 @@ size_t list_scratch_ctas(long long W);
 // update_radiance's list (internal_render.cpp:1142-1168) built on the device from the int16
 // grid: rule-listed blocks in scan order, then the specials not already listed, in order.
 // out holds W + n_specials entries; *count (device) receives the list length.
+// dependent: the stream's previous kernel does not write the grid, and this may start in its tail.
 cudaError_t launch_update_list(const int16_t* grid, int X, int Y, int Z, const short4* specials, int n_specials,
-                               const ListScratch& scratch, short4* out, int* count, cudaStream_t stream);
+                               const ListScratch& scratch, short4* out, int* count, bool dependent, cudaStream_t stream);
 
 // Probes within Chebyshev distance `radius` of the edited blocks (edits as (x, y, z, block), all
 // inside the world), in scan order, into out (W entries); *count (device) receives the length.
@@ -248,16 +249,31 @@ struct MapArgs {
 };
 // exec_copies' static-to-temporary block copies: (src slot, dst slot) pairs.
 cudaError_t launch_palette_copies(uint8_t* pal, const int2* copies, int n, cudaStream_t stream);
-// map.comp for mesh `mesh` (model voxels x-fastest, mx*my*mz bytes): each write is claimed in
-// owner (one 64-bit word per voxel of the palette slots from static_blocks up, zero at the start
-// of a frame); launch_map_resolve then writes the winners into those slots.
-cudaError_t launch_map(const int16_t* grid, int X, int Y, int Z, int n_slots, int static_blocks, const uint8_t* model,
-                       int mx, int my, int mz, const MapArgs& a, int mesh, unsigned long long* owner,
-                       cudaStream_t stream);
+// map.comp for n meshes, the first of them mesh number `first` of the frame (voxels x-fastest,
+// size[0]*size[1]*size[2] bytes each): each write is claimed in owner (one 64-bit word per voxel of the
+// palette slots from static_blocks up, zero at the start of a frame); launch_map_resolve then writes
+// the winners into those slots.
+struct MapMesh {
+    MapArgs a;
+    const uint8_t* voxels;
+    int size[3];
+};
+cudaError_t launch_map(const int16_t* grid, int X, int Y, int Z, int n_slots, int static_blocks, const MapMesh* meshes,
+                       int n, int first, unsigned long long* owner, cudaStream_t stream);
 cudaError_t launch_map_resolve(uint8_t* pal_tmp, const unsigned long long* owner, size_t n, cudaStream_t stream);
 // Occupancy masks (128 words per compact id) from the device palette; slot_of[c] = -1: empty.
 cudaError_t launch_compact_bits(const uint8_t* pal, const int* slot_of, int n_compact, uint32_t* cbits,
                                 cudaStream_t stream);
+
+// One changed block of a context's world: its new id and compact id (read by the kernel from
+// page-locked memory).
+struct CellEdit {
+    uint32_t index;              // x + X*(y + Y*z)
+    int16_t block;
+    uint16_t compact;
+};
+cudaError_t launch_apply_cells(const CellEdit* edits, int n, int16_t* grid, void* cgrid, bool wide, int X, int Y,
+                               cudaStream_t stream);
 
 // One block edit of a served world: worlds[world].grid[index] = block and its compact id.
 struct EditRecord {

@@ -1021,7 +1021,10 @@ int lumrad_server_add_world(LumRadServer server, LumRadContext world, int* id) {
     LUMRAD_TRY(cudaSetDevice(sv->s.device));
     LUMRAD_TRY(cudaStreamSynchronize(c->stream));
     DeviceWorld& dw = c->world;
-    if (!dw.h_cur.empty()) dw.grid_dirty = true;   // a blockified frame is dropped: edits apply to the loaded world
+    // a blockified frame is dropped: edits apply to the loaded world; and the upload is waited for (the
+    // launches run on other streams)
+    if (!dw.h_cur.empty() || !dw.edited.empty()) dw.grid_dirty = true;
+    dw.origin_end = -1;   // the server's edits change the grid
     int rc = dw.sync_inputs(c->stream);
     if (rc) return rc;
     if ((rc = prepare_world(dw, c->stream))) return rc;

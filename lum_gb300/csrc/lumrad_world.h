@@ -96,6 +96,17 @@ struct DeviceWorld {
     std::map<int, float4*> d_dirs;
     // blockify: the frame's grid with temporary blocks (empty when not blockified)
     std::vector<int16_t> h_cur;
+    std::vector<uint32_t> blk_cells;      // the blocks in which h_cur differs from h_grid
+    int origin_end = -1;                  // one past the highest block id of h_grid, or more (-1: not known)
+    // blocks of h_grid changed since its upload, while neither grid_dirty nor compact_dirty: applied
+    // one by one (apply_cells) instead of uploading and renumbering the whole world
+    std::vector<uint32_t> edited;
+    // apply_cells' records, page-locked and read by the kernel: two halves, each with the event after
+    // its last kernel
+    CellEdit* h_cells[2] = {nullptr, nullptr};
+    size_t cells_cap[2] = {0, 0};
+    cudaEvent_t ev_cells[2] = {nullptr, nullptr};
+    int cells_half = 0;
     // one past the highest palette slot that may hold non-zero voxels on the device (blockify
     // clears the temporary slots up to here); every slot after a palette upload
     int pal_dirty_end = 1 << 30;
@@ -120,6 +131,12 @@ struct DeviceWorld {
     // Device bytes this world holds.
     size_t footprint() const;
     int sync_inputs(cudaStream_t stream);
+    // The n blocks at idx (repeats allowed) into the device's grid and compact grid, with their ids of
+    // g; ids new to the world get compact ids, their slots uploaded, and with host_bits their masks
+    // from the host palette.  *fits false: one of them needs a wider compact grid, nothing launched.
+    int apply_cells(const uint32_t* idx, size_t n, const int16_t* g, bool host_bits, cudaStream_t stream, bool* fits);
+    // room for the masks and slots of the world's compact ids, and of every id that has a palette slot
+    int ensure_compact_room(cudaStream_t stream);
     int ensure_dirs(int R, cudaStream_t stream, const float4** out);
     int ensure_scratch(size_t groups, int R, cudaStream_t stream);
     int ensure_hits(size_t n);
@@ -156,6 +173,7 @@ struct Context {
     long long api_calls = 0;
     long long pass_mark = -1;
     long long uploads_mark = -1;
+    long long list_uploads = -1;            // world.uploads at the last device list
 
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_req = nullptr;
@@ -199,11 +217,11 @@ struct Context {
     std::vector<Model> models;
     unsigned long long* d_map_owner = nullptr;   // one word per voxel of the temporary palette slots
     size_t map_owner_cap = 0;
-    // blockify staging, page-locked so the frame's uploads do not block the host: the working
-    // grid (W int16), compact grid (uint16 at most), compact slots (n_slots + 128 ints) and
-    // palette copies (n_slots int2); and the copies' device buffer
-    uint8_t* h_blk = nullptr;
-    int2* d_blk_copies = nullptr;
+    // blockify staging: the palette copies (n_slots int2 each), page-locked and read by the kernel; two
+    // halves, each with the event after its last kernel
+    int2* h_blk[2] = {nullptr, nullptr};
+    cudaEvent_t ev_blk[2] = {nullptr, nullptr};
+    int blk_half = 0;
     // device update-list builder
     ListScratch list{};
     short4* d_specials = nullptr;

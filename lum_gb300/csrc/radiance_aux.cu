@@ -477,38 +477,68 @@ __global__ void __launch_bounds__(256) palette_copy_kernel(uint8_t* __restrict__
 // one after another in linear order (x fastest) and the meshes in order: each invocation
 // atomicMax-es (mesh, invocation, value) into the target's 64-bit owner word; a resolve pass
 // writes the winning values.
-__global__ void map_kernel(const int16_t* __restrict__ grid, int X, int Y, int Z, int n_slots, int static_blocks,
-                           const uint8_t* __restrict__ model, int mx, int my, int mz, MapArgs a,
-                           unsigned long long* __restrict__ owner, unsigned long long mesh_key) {
-    const int gx = blockIdx.x * blockDim.x + threadIdx.x;
-    const int gy = blockIdx.y * blockDim.y + threadIdx.y;
-    const int gz = blockIdx.z * blockDim.z + threadIdx.z;
-    if (gx >= a.dims[0] || gy >= a.dims[1] || gz >= a.dims[2]) return;
+//
+// One launch covers up to kMapMeshes meshes (a frame's eight took eight launches of about 3.7 us, most
+// of it latency): group g of mesh k is CTA group0[k] + g, its 4x4x4 invocations the CTA's threads.
+constexpr int kMapMeshes = 24;
+struct MapBatch {
+    MapMesh mesh[kMapMeshes];
+    unsigned group0[kMapMeshes + 1];
+    int n, first;
+};
+static_assert(sizeof(MapBatch) <= 3584, "kernel parameters");
+__global__ void __launch_bounds__(64)
+map_kernel(const int16_t* __restrict__ grid, int X, int Y, int Z, int n_slots, int static_blocks,
+           const __grid_constant__ MapBatch batch, unsigned long long* __restrict__ owner) {
+    int k = 0;
+    while (blockIdx.x >= batch.group0[k + 1]) k++;
+    const MapArgs& a = batch.mesh[k].a;
+    const unsigned gw = (unsigned)a.dims[0] / 4u, gh = (unsigned)a.dims[1] / 4u;
+    const unsigned group = blockIdx.x - batch.group0[k], gq = group / gw;
+    const int gx = (int)(4u * (group - gq * gw) + (threadIdx.x & 3u));
+    const int gy = (int)(4u * (gq % gh) + ((threadIdx.x >> 2) & 3u));
+    const int gz = (int)(4u * (gq / gh) + (threadIdx.x >> 4));
+    const int mx = batch.mesh[k].size[0], my = batch.mesh[k].size[1], mz = batch.mesh[k].size[2];
     // world_voxel = vec3(g) / 1.0 + vec3(0.5) + vec3(shift)   (:37-40)
     const float wx = fadd(fadd((float)gx, 0.5f), (float)a.shift[0]);
     const float wy = fadd(fadd((float)gy, 0.5f), (float)a.shift[1]);
     const float wz = fadd(fadd((float)gz, 0.5f), (float)a.shift[2]);
     const int ix = f2i(wx), iy = f2i(wy), iz = f2i(wz);   // (:41)
-    // model_voxel = (inverse_trans * vec4(world_voxel, 1)).xyz, columns summed in order   (:47-48)
-    const float* m = a.inv;   // column-major m[4*col + row]
-    const float vx = fadd(fadd(fadd(fmul(m[0], wx), fmul(m[4], wy)), fmul(m[8], wz)), m[12]);
-    const float vy = fadd(fadd(fadd(fmul(m[1], wx), fmul(m[5], wy)), fmul(m[9], wz)), m[13]);
-    const float vz = fadd(fadd(fadd(fmul(m[2], wx), fmul(m[6], wy)), fmul(m[10], wz)), m[14]);
-    const int px = f2i(vx), py = f2i(vy), pz = f2i(vz);
     // target block = iworld / 16 (OpSDiv); out of range reads block 0   (:50-52)
     const int bx = ix / 16, by = iy / 16, bz = iz / 16;
     int id = 0;
     if (bx >= 0 && by >= 0 && bz >= 0 && bx < X && by < Y && bz < Z)
         id = grid[(size_t)bx + (size_t)X * ((size_t)by + (size_t)Y * bz)];
     if (id < static_blocks || id >= n_slots) return;   // (:59); the palette ends at its last slot
+    // model_voxel = (inverse_trans * vec4(world_voxel, 1)).xyz, columns summed in order   (:47-48)
+    const float* m = a.inv;   // column-major m[4*col + row]
+    const float vx = fadd(fadd(fadd(fmul(m[0], wx), fmul(m[4], wy)), fmul(m[8], wz)), m[12]);
+    const float vy = fadd(fadd(fadd(fmul(m[1], wx), fmul(m[5], wy)), fmul(m[9], wz)), m[13]);
+    const float vz = fadd(fadd(fadd(fmul(m[2], wx), fmul(m[6], wy)), fmul(m[10], wz)), m[14]);
+    const int px = f2i(vx), py = f2i(vy), pz = f2i(vz);
     int v = 0;
     if (px >= 0 && py >= 0 && pz >= 0 && px < mx && py < my && pz < mz)
-        v = model[(size_t)px + (size_t)mx * ((size_t)py + (size_t)my * pz)];   // (:60)
+        v = batch.mesh[k].voxels[(size_t)px + (size_t)mx * ((size_t)py + (size_t)my * pz)];   // (:60)
     if (v == 0) return;
     const unsigned long long lin =
         (unsigned long long)gx + (unsigned long long)a.dims[0] * ((unsigned long long)gy + (unsigned long long)a.dims[1] * gz);
     const size_t t = ((size_t)(id - static_blocks) << 12) | (smod(iz, 16) << 8) | (smod(iy, 16) << 4) | smod(ix, 16);
+    const unsigned long long mesh_key = (unsigned long long)(batch.first + k + 1) << 40;
     atomicMax(owner + t, mesh_key | (lin << 8) | (unsigned long long)v);   // (:54,62)
+}
+
+// Changed blocks of a context's world into its grid and compact grid (a block listed twice has the same
+// value both times).
+__global__ void apply_cells_kernel(const CellEdit* __restrict__ edits, int n, int16_t* __restrict__ grid, void* cgrid, int wide,
+                                   int X, int Y) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const CellEdit e = edits[k];
+    const unsigned q = e.index / (unsigned)X;
+    const size_t cell = (e.index - q * (unsigned)X) + (size_t)(X + 1) * (q % (unsigned)Y + (size_t)(Y + 1) * (q / (unsigned)Y));
+    grid[e.index] = e.block;
+    if (wide) static_cast<uint16_t*>(cgrid)[cell] = e.compact;
+    else static_cast<uint8_t*>(cgrid)[cell] = (uint8_t)e.compact;
 }
 
 __global__ void map_resolve_kernel(uint8_t* __restrict__ pal_tmp, const unsigned long long* __restrict__ owner,
@@ -594,14 +624,33 @@ cudaError_t launch_palette_copies(uint8_t* pal, const int2* copies, int n, cudaS
     return cudaGetLastError();
 }
 
-cudaError_t launch_map(const int16_t* grid, int X, int Y, int Z, int n_slots, int static_blocks, const uint8_t* model,
-                       int mx, int my, int mz, const MapArgs& a, int mesh, unsigned long long* owner,
-                       cudaStream_t stream) {
-    if (a.dims[0] <= 0 || a.dims[1] <= 0 || a.dims[2] <= 0) return cudaSuccess;
-    const dim3 block(4, 4, 4);   // local_size 4x4x4 (:32)
-    const dim3 grid_dim((a.dims[0] + 3) / 4, (a.dims[1] + 3) / 4, (a.dims[2] + 3) / 4);
-    map_kernel<<<grid_dim, block, 0, stream>>>(grid, X, Y, Z, n_slots, static_blocks, model, mx, my, mz, a, owner,
-                                               (unsigned long long)(mesh + 1) << 40);
+cudaError_t launch_map(const int16_t* grid, int X, int Y, int Z, int n_slots, int static_blocks, const MapMesh* meshes,
+                       int n, int first, unsigned long long* owner, cudaStream_t stream) {
+    for (int i = 0; i < n;) {   // as many meshes as fit a launch (2^31 groups, kMapMeshes)
+        MapBatch batch;
+        batch.n = 0;
+        batch.first = first + i;
+        batch.group0[0] = 0;
+        unsigned long long groups = 0;
+        for (; i < n && batch.n < kMapMeshes; i++) {
+            const int* d = meshes[i].a.dims;
+            const bool empty = d[0] <= 0 || d[1] <= 0 || d[2] <= 0;
+            const unsigned long long g = empty ? 0 : (unsigned long long)(d[0] / 4) * (d[1] / 4) * (d[2] / 4);   // local_size 4x4x4 (:32)
+            if (groups + g >= 1ull << 31) break;
+            groups += g;
+            batch.mesh[batch.n] = meshes[i];
+            batch.group0[++batch.n] = (unsigned)groups;
+        }
+        if (batch.n == 0) return cudaErrorInvalidValue;   // (a mesh covers fewer than 2^32 voxels)
+        if (groups > 0) map_kernel<<<(unsigned)groups, 64, 0, stream>>>(grid, X, Y, Z, n_slots, static_blocks, batch, owner);
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_apply_cells(const CellEdit* edits, int n, int16_t* grid, void* cgrid, bool wide, int X, int Y,
+                               cudaStream_t stream) {
+    if (n <= 0) return cudaSuccess;
+    apply_cells_kernel<<<(n + 127) / 128, 128, 0, stream>>>(edits, n, grid, cgrid, wide ? 1 : 0, X, Y);
     return cudaGetLastError();
 }
 
@@ -620,10 +669,10 @@ cudaError_t launch_compact_bits(const uint8_t* pal, const int* slot_of, int n_co
 }
 
 cudaError_t launch_update_list(const int16_t* grid, int X, int Y, int Z, const short4* specials, int n_specials,
-                               const ListScratch& s, short4* out, int* count, cudaStream_t stream) {
+                               const ListScratch& s, short4* out, int* count, bool dependent, cudaStream_t stream) {
     const long long W = (long long)X * Y * Z;
     const int ctas = (int)((W + kListCta - 1) / kListCta);
-    cudaError_t e = launch_kernel(list_flags_kernel, ctas, kListCta, 0, stream, true, grid, X, Y, Z, (unsigned)W, s.bits, s.cta_counts);
+    cudaError_t e = launch_kernel(list_flags_kernel, ctas, kListCta, 0, stream, dependent, grid, X, Y, Z, (unsigned)W, s.bits, s.cta_counts);
     if (e != cudaSuccess) return e;
     if ((e = launch_list_write(s, X, Y, W, out, count, n_specials > 0 ? s.listed : nullptr, stream)) != cudaSuccess) return e;
     if (n_specials > 0) list_specials_kernel<<<1, kScanCta, 0, stream>>>(specials, n_specials, s.bits, X, Y, s.listed, out, count);
