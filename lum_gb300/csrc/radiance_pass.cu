@@ -593,6 +593,7 @@ struct FinShared {
     uint8_t hit[kFinWarps * kTaskRays];
     int n_hits;
     unsigned lookups;
+    int irregular;               // whether a hit's ray is not regular
     __device__ __forceinline__ void put_light(int task, int lane, float3 v) {
         float* s = light + task * kFinStride + lane;
         s[0] = v.x;
@@ -602,6 +603,23 @@ struct FinShared {
 };
 static_assert(kFinWarps * kTaskRays <= 256 && 3 * kFinWarps <= 32 && (kFinWarps & (kFinWarps - 1)) == 0,
               "ray numbers fit 8 bits, one lane per channel and task");
+
+// A hit ray by the general forms, its light into the CTA's; returns its lookups.  (Out of line, and with
+// nothing of the caller's passed by address: the regular rays' path keeps its values in registers.)
+template <class Store, bool RECORD>
+__device__ __noinline__ uint32_t finalize_general(const WorldPass& w, const RayBuffer& rays, const int* ray_blk, int idx, int ray,
+                                                  long long gr, FinShared& sh) {
+    const uint2 res = rays.res[idx];
+    const float4 od = rays.od[idx];
+    const float2 dd = rays.dd[idx];
+    float3 u;
+    float4 m;
+    const uint32_t n = refine_general<RECORD>(w, make_float3(od.x, od.y, od.z), make_float3(od.w, dd.x, dd.y), __uint_as_float(res.x),
+                                              res.y, RECORD ? __ldcg(ray_blk + idx) : 0, gr, u, m);
+    grid_dependency_wait();
+    sh.put_light(ray >> 5, ray & 31, shade_hit<Store>(w, u, m));
+    return n;
+}
 
 // Warps per CTA, and CTAs per SM of the lean and the general form.  The kernel waits on its chain of
 // dependent lookups and its barriers, so small CTAs pay: two warps for a group's eight tasks, 24 CTAs
@@ -635,6 +653,7 @@ __device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, 
     if (threadIdx.x == 0) {
         sh.n_hits = 0;
         sh.lookups = 0;
+        sh.irregular = 0;
     }
     __syncthreads();
     const int t0 = la.chunk_begin + group * kFinWarps;   // worlds start at multiples of 8
@@ -662,6 +681,7 @@ __device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, 
         base = __shfl_sync(kFull, base, 0);
         if (hit) {
             sh.hit[base + __popc(hm & ((1u << lane) - 1u))] = (uint8_t)(k * kTaskRays + lane);
+            if (!(res.y & kInfoRegular)) sh.irregular = 1;
         } else {
             sh.put_light(k, lane, sky_light(make_float3(od.w, dd.x, dd.y)));
             if (RECORD)
@@ -673,25 +693,29 @@ __device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, 
     // scheduler of the SM gets its share)
     const int n_hits = sh.n_hits;
 #pragma unroll 1
-    for (int j = (int)(threadIdx.x + 32 * (group % CW)) % (32 * CW); j < n_hits; j += 32 * CW) {
+    for (int j = (int)(threadIdx.x + 32 * (group % CW)) % (32 * CW); !RECORD && j < n_hits; j += 32 * CW) {
         const int ray = sh.hit[j], idx = first + ray;
         const uint2 res = la.rays.res[idx];
+        if (!(res.y & kInfoRegular)) continue;   // below
         const float4 od = la.rays.od[idx];
         const float2 dd = la.rays.dd[idx];
         const float3 o = make_float3(od.x, od.y, od.z), d = make_float3(od.w, dd.x, dd.y);
         const float frac = __uint_as_float(res.x);
         float3 u;
         float4 m;
-        if (RECORD) {
-            lookups += refine_general<true>(*wp, o, d, frac, res.y, __ldcg(la.ray_blk + idx), (long long)t0_local * kTaskRays + ray, u, m);
-        } else if (res.y & kInfoRegular) {
-            const MarchView mv = march_view(*wp);
-            lookups += mv.wide ? refine_regular<true>(*wp, mv, o, d, frac, u, m) : refine_regular<false>(*wp, mv, o, d, frac, u, m);
-        } else {
-            lookups += refine_irregular(*wp, o, d, frac, u, m);
-        }
+        const MarchView mv = march_view(*wp);
+        lookups += mv.wide ? refine_regular<true>(*wp, mv, o, d, frac, u, m) : refine_regular<false>(*wp, mv, o, d, frac, u, m);
         grid_dependency_wait();   // from here on the volumes: the previous pass's launch has finished
         sh.put_light(ray >> 5, ray & 31, shade_hit<Store>(*wp, u, m));
+    }
+    // the hits of rays that are not regular (apart, so that the loop above has no call to keep values
+    // for), or every hit if they are recorded
+    if (RECORD || sh.irregular) {
+        for (int j = threadIdx.x; j < n_hits; j += 32 * CW) {
+            const int ray = sh.hit[j], idx = first + ray;
+            if (RECORD || !(la.rays.res[idx].y & kInfoRegular))
+                lookups += finalize_general<Store, RECORD>(*wp, la.rays, la.ray_blk, idx, ray, (long long)t0_local * kTaskRays + ray, sh);
+        }
     }
     lookups = __reduce_add_sync(kFull, lookups);
     if (lane == 0 && lookups) atomicAdd(&sh.lookups, lookups);

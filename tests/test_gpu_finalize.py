@@ -33,16 +33,16 @@ def test_pass_bits(dims, rays):
     _run(w, req, rays=rays, max_dist=128.0, blend=0.1, time_seed=9)
 
 
-@pytest.mark.parametrize("size,shift", [(1, 0), (3, 2)])
-def test_odd_worlds(size, shift):
-    dims = (11, 9, 6)
+@pytest.mark.parametrize("dims,size,shift", [((11, 9, 6), 1, 0), ((11, 9, 6), 3, 2), ((48, 44, 11), 1, 0)])
+def test_odd_worlds(dims, size, shift):
     w = worldgen.terrain_world(dims, seed=42, extra_blocks=60)
     w.palette[0] = (worldgen.uniform(1, 2, 4096) < 0.002).reshape(16, 16, 16) * 5   # voxels in "air"
     g = w.grid.reshape(-1)
     g[worldgen.randint(3, 4, 30, 0, g.size)] = -worldgen.randint(5, 6, 30, 1, 70).astype(np.int16)
     g[worldgen.randint(7, 8, 10, 0, g.size)] = 900
     req = worldgen.all_probes(dims)
-    outside = np.array([[-1, 2, 2, 0], [11, 3, 3, 0], [4, -2, 1, 0], [4, 9, 1, 0], [5, 5, 6, 0], [5, 5, -1, 0],
+    X, Y, Z = dims
+    outside = np.array([[-1, 2, 2, 0], [X, 3, 3, 0], [4, -2, 1, 0], [4, Y, 1, 0], [5, 5, Z, 0], [5, 5, -1, 0],
                         [-300, 7, 2, 0], [30000, -30000, 12, 0]], np.int16)
     req = np.concatenate([req[:50], outside[:4], req[50:], outside[4:]])
     _run(w, req, rays=64, max_dist=96.0, blend=0.2, time_seed=3, size=size, shift=shift)
