@@ -6,13 +6,12 @@
 //   march_kernel     persistent warps take tasks from a queue in guided chunks (large early,
 //                    single tasks at the end; through a shared-memory block per CTA when the
 //                    launch has few tasks per warp).  A warp sets up a task's 32 rays in lock step
-//                    (hash seeds, direction, origin, 1/direction) into a 32-ray ring in shared
-//                    memory, takes their first coarse step there (38% of the demo's rays end on
-//                    it) and puts the rest into the ring.  Its lanes march in a flat loop, up to
-//                    three coarse steps per iteration; a lane whose ray ends writes its result
-//                    (fraction, info; the set-up wrote its origin and direction) and takes the next
-//                    ray in ring order.  The ring is set up again as soon as its rays are handed
-//                    out, so lanes never wait for each other.
+//                    (hash seeds, direction, origin, 1/direction), the rays its lanes were marching
+//                    in a pool in shared memory meanwhile, and takes their first coarse step there
+//                    (38% of the demo's rays end on it).  Its lanes march in a flat loop, up to three
+//                    coarse steps per iteration; a lane whose ray ends writes its result (fraction,
+//                    info; the set-up wrote its origin and direction) and takes a ray from the pool;
+//                    when that is empty, the next task is set up, so lanes never wait for each other.
 //   finalize_kernel  eight consecutive tasks per CTA of two warps: the rays read back, the hits
 //                    packed 32 to a warp for the refine DDA, material, trilinear fetch of the
 //                    previous radiance and shading; then one lane per task and channel for the
@@ -79,10 +78,10 @@ __device__ __forceinline__ float exit_fraction(float3 o, float3 d, float rx, flo
 // STAGE: one CTA of kStageWarps warps per SM, with the launch's compact world (compact grid and
 // occupancy masks, every world of the launch the same) copied into shared memory at the start;
 // lookups are then 32-bit-addressed shared loads (fewer address instructions, lower latency than
-// the L1-resident form: 8% off the demo step's march when it was introduced).  Used where the world fits beside the rays'
-// rings and parking space (98 KB of the 227 KB per CTA: a 64x64x16 world of 34 block types takes
-// 81 KB, and compact worlds up to ~125 KB fit); other launches (batches, servers, larger worlds,
-// hit records) read the world from global memory through L1.
+// the L1-resident form: a pass over every probe of a 64x64x32 world, 256 rays, 1,979 -> 1,764 us once its
+// 157 KB fit; 8% off the demo step's march).  Used where the world fits beside the rays' pools (52 KB of the 227 KB per CTA: a 64x64x16 world of 34 block types takes 87 KB, and compact
+// worlds up to 174 KB fit); other launches (batches, servers, larger worlds, hit records) read the
+// world from global memory through L1.
 constexpr int kStageWarps = 32;
 // Queue defaults (LaunchArgs guided_div / max_chunk = 0): the CTA queue's divisor and the chunk
 // cap; the per-warp queue divides by kWarpQueueDiv
@@ -92,11 +91,17 @@ static_assert(LUMRAD_MAX_CHUNK < (1 << 12) && kQueueCap <= LUMRAD_MAX_CHUNK, "a 
 constexpr int kWarpQueueDiv = 1;
 // launches with fewer tasks than this per warp claim through the CTA queue (march_kernel's CTAQ)
 constexpr int kCtaQueueTasksPerWarp = 32;
-// A warp's shared-memory ring holds the rays of one task (origin + ray index, direction + fraction,
-// 1/direction + exit fraction) that wait while the lanes march the previous ones; the next task is
-// set up once they are all handed out.  (Rings of two and four tasks: 3% and 11-12% slower on a
-// single pass, their shared memory costs a CTA per SM.)
-constexpr size_t kStageRingBytes = (size_t)kStageWarps * 6 * kTaskRays * sizeof(float4);
+// A warp's pool: the rays its lanes were marching when the next task was set up (the set-up needs
+// their registers; the new task's rays that go on stay in the lanes that built them).  Idle lanes take
+// from it, and when it is empty the next task is set up.  A ray: origin + index, direction + fraction,
+// 1/direction + exit fraction, steps.  (Against a ring that the new task's rays all went through and a
+// second place for the lanes': half the shared memory, 371 -> 339 M warp instructions for a run of 64
+// worlds batched, 2,229 -> 2,189 us with its reads; the 64-ray demo frame 178 -> 170 us.)
+struct RayPool {
+    float4 o[kTaskRays], d[kTaskRays], i[kTaskRays];
+    int steps[kTaskRays];
+};
+constexpr size_t kStagePoolBytes = (size_t)kStageWarps * sizeof(RayPool);
 
 // Tasks are claimed in two levels.  A CTA takes guided blocks from the launch's queue word
 // (remaining / (div * CTAs), clamped to [1, cap * warps per CTA]) into a shared-memory block word
@@ -180,9 +185,9 @@ __device__ __noinline__ long long refill_block(const LaunchArgs& la, int n_round
 }
 
 // What bounds it: instruction issue (84% of the slots on the demo's 8-pass launch, every world
-// lookup in shared memory).  Per 32-ray task that launch issues 912 warp instructions, of which the
-// set-up with its first step is about 350 and an iteration (3 steps of about 45 and the hand-out)
-// 200.  The launch: 436 -> 373 us, 452 -> 383 M warp instructions, with: lookups without range
+// lookup in shared memory).  Per 32-ray task that launch issues 897 warp instructions, of which the
+// set-up with its first step is about 400 and an iteration (3 steps of about 45 and the hand-out)
+// 200.  The launch: 436 -> 371 us, 452 -> 376 M warp instructions, with: lookups without range
 // tests or conversions for regular rays (solid_inside), x and y in register pairs, the first step
 // in the set-up, results and hand-outs once per three steps, and reciprocals and the square root
 // without their checks for operands that cannot occur.
@@ -202,15 +207,13 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
             }
         }
     }
-    float4 (*s_ray)[3][kTaskRays];    // the ring
-    float4 (*s_park)[3][kTaskRays];   // in-flight ray state while the warp sets up
+    RayPool* s_pool;
     const uint8_t* s_cg = nullptr;
     const uint16_t* s_rows = nullptr;
     if constexpr (STAGE) {
         extern __shared__ __align__(16) unsigned char s_dyn[];
-        s_ray = reinterpret_cast<float4 (*)[3][kTaskRays]>(s_dyn);
-        s_park = reinterpret_cast<float4 (*)[3][kTaskRays]>(s_dyn + (size_t)kStageWarps * 3 * kTaskRays * sizeof(float4));
-        unsigned char* wb = s_dyn + kStageRingBytes;
+        s_pool = reinterpret_cast<RayPool*>(s_dyn);
+        unsigned char* wb = s_dyn + kStagePoolBytes;
         const WorldPass& w0 = la.worlds ? la.worlds[0] : la.single;
         const int cg_bytes = (w0.X + 1) * (w0.Y + 1) * (w0.Z + 1) * (w0.cgrid_wide ? 2 : 1);
         const int cg_pad = (cg_bytes + 15) & ~15;
@@ -225,10 +228,8 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
         s_cg = wb;
         s_rows = reinterpret_cast<const uint16_t*>(wb + cg_pad);
     } else {
-        __shared__ float4 a_ray[kWarps][3][kTaskRays];
-        __shared__ float4 a_park[kWarps][3][kTaskRays];
-        s_ray = a_ray;
-        s_park = a_park;
+        __shared__ RayPool a_pool[kWarps];
+        s_pool = a_pool;
     }
 
     if (la.dev_count) grid_dependency_wait();   // a list from the kernels before (the world is in place by now)
@@ -260,9 +261,7 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    float4* so = s_ray[wib][0];
-    float4* sd = s_ray[wib][1];
-    float4* si = s_ray[wib][2];
+    RayPool& pool = s_pool[wib];
     const unsigned lt_mask = (1u << lane) - 1u;
     // current world (warp-uniform)
     const WorldPass* wp = &la.single;
@@ -271,10 +270,8 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
     unsigned kb = 0;
     int max_steps = 0;
     int w_begin = 0, w_end = 0;
-    // the ring: rays [issued, loaded) of the last task set up wait to be handed out; ring_fast: all
-    // of them are regular
-    int issued = 0, loaded = 0;
-    bool ring_fast = true;
+    int taken = 0, pooled = 0;   // the pool's rays [taken, pooled) wait for a lane
+    bool slow = false;           // a ray of the lanes or the pool is not regular
     int tb = 0, te = 0;          // grabbed task chunk [tb, te)
     bool exhausted = false;
     int pending = -1;            // grabbed task of another world, waiting for the lanes to drain
@@ -324,21 +321,21 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
         cxy = pack2(dx > 0.0f ? 16.0f - kBlockBias : -kBlockBias, dy > 0.0f ? 16.0f - kBlockBias : -kBlockBias);
         cz = dz > 0.0f ? 16.0f - kBlockBias : -kBlockBias;
     };
-    // hand the next rays in ring order to the lanes in `need`
+    // the pool's next rays to the lanes in `need`
     auto assign = [&](unsigned need) {
-        const int slot = issued + __popc(need & lt_mask);
-        if (((need >> lane) & 1u) && slot < loaded) {
-            const float4 o4 = so[slot], d4 = sd[slot], i4 = si[slot];
-            my = __float_as_int(o4.w);   // the ray's round-relative index, stored with its origin
+        const int slot = taken + __popc(need & lt_mask);
+        if (((need >> lane) & 1u) && slot < pooled) {
+            const float4 o4 = pool.o[slot], d4 = pool.d[slot], i4 = pool.i[slot];
+            my = __float_as_int(o4.w);
             oxy = pack2(o4.x, o4.y); oz = o4.z;
             dxy = pack2(d4.x, d4.y); dz = d4.z;
             ivxy = pack2(i4.x, i4.y); ivz = i4.z;
             fexit = i4.w;
             corner(d4.x, d4.y);
             frac = d4.w;
-            steps = d4.w != 0.0f ? 1 : 0;   // a first step in the set-up leaves at least 0.5
+            steps = pool.steps[slot];
         }
-        issued = min(loaded, issued + __popc(need));
+        taken = min(pooled, taken + __popc(need));
     };
     // ray i has ended, its last lookup at p
     auto end_ray = [&](int i, float px, float py, float pz, bool solid, uint32_t info) {
@@ -382,8 +379,8 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
 
     // The coarse march of the lanes' rays, up to three steps per iteration (two: 1-2% slower, four:
     // equal): a lane whose ray ends takes no further one, and the ended rays' results are written
-    // and their lanes given new rays once per iteration.  Runs until the ring is empty while tasks
-    // may remain, or no lane has a ray.  FAST: every lane's ray and the ring's are regular.
+    // and their lanes given new rays once per iteration.  Runs until the pool is empty while tasks
+    // may remain, or no lane has a ray.  FAST: every lane's ray and the pool's are regular.
     auto march = [&](auto fast_tag, auto wide_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
         constexpr bool WIDE = decltype(wide_tag)::value;
@@ -440,24 +437,34 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
             const unsigned fm = __ballot_sync(kFull, fin);
             if (fm) {
                 assign(fm);
-                if (loaded == issued && (more_tasks() || !__any_sync(kFull, my >= 0))) break;
+                if (taken == pooled && (more_tasks() || !__any_sync(kFull, my >= 0))) break;
             }
         }
     };
 
     while (true) {
-        // 1. set up tasks until one leaves rays in the ring
-        const bool refill = loaded == issued && (pending >= 0 || more_tasks());
-        if (refill && my >= 0) {   // park: the set-up needs the registers
-            float x, y;
-            unpack2(oxy, x, y);
-            s_park[wib][0][lane] = make_float4(x, y, oz, frac);
-            unpack2(dxy, x, y);
-            s_park[wib][1][lane] = make_float4(x, y, dz, __int_as_float(steps));
-            unpack2(ivxy, x, y);
-            s_park[wib][2][lane] = make_float4(x, y, ivz, fexit);
+        // 1. the pool empty: set up tasks until one leaves rays
+        const bool refill = taken == pooled && (pending >= 0 || more_tasks());
+        bool left = !refill;
+        if (refill) {   // the lanes' rays into the pool: the set-up needs the registers
+            const unsigned pm = __ballot_sync(kFull, my >= 0);
+            slow = __any_sync(kFull, my >= 0 && fexit < 0.0f);
+            taken = 0;
+            pooled = __popc(pm);
+            if (my >= 0) {
+                const int slot = __popc(pm & lt_mask);
+                float x, y;
+                unpack2(oxy, x, y);
+                pool.o[slot] = make_float4(x, y, oz, __int_as_float(my));
+                unpack2(dxy, x, y);
+                pool.d[slot] = make_float4(x, y, dz, frac);
+                unpack2(ivxy, x, y);
+                pool.i[slot] = make_float4(x, y, ivz, fexit);
+                pool.steps[slot] = steps;
+                my = -1;
+            }
         }
-        while (refill && loaded == issued) {
+        while (!left) {
             const int t = next_task();
             if (t < 0) break;
             if (t < w_begin || t >= w_end) {
@@ -470,7 +477,7 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
                 // compact world with the same bound (passes of one context), whose rays march alike
                 const bool alike = reinterpret_cast<const uint8_t*>(wq->cgrid) == mv.cgrid &&
                                    wq->max_dist == max_dist;
-                if (!alike && __any_sync(kFull, my >= 0)) {
+                if (!alike && pooled > 0) {
                     if (pending != t) tb++;
                     pending = t;
                     break;
@@ -501,7 +508,7 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
                 ry = __frcp_rn(d.y);
                 rz = __frcp_rn(d.z);
             }
-            // the rays' first step here, where all 32 lanes take it; the rays that go on into the ring
+            // the rays' first step here, where all 32 lanes take it
             oxy = pack2(o.x, o.y); oz = o.z;
             dxy = pack2(d.x, d.y); dz = d.z;
             ivxy = pack2(rx, ry); ivz = rz;
@@ -509,45 +516,30 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
             corner(d.x, d.y);
             frac = 0.0f;
             steps = 0;
-            bool on = true;
-            ring_fast = __all_sync(kFull, regular);
-            if (ring_fast && step(mv.wide) && ray_ended()) {
+            my = idx;
+            const bool fast = __all_sync(kFull, regular);
+            if (!fast) slow = true;
+            else if (step(mv.wide) && ray_ended()) {
                 end_ray(idx, px, py, pz, solid, hit_info());
-                on = false;
+                my = -1;
             }
-            const unsigned sm = __ballot_sync(kFull, on);
-            if (on) {
-                const int slot = __popc(sm & lt_mask);
-                so[slot] = make_float4(o.x, o.y, o.z, __int_as_float(idx));
-                sd[slot] = make_float4(d.x, d.y, d.z, frac);
-                si[slot] = make_float4(rx, ry, rz, fexit);
-            }
-            issued = 0;
-            loaded = __popc(sm);
+            left = __any_sync(kFull, my >= 0);
         }
         __syncwarp();
-        if (refill && my >= 0) {
-            const float4 a = s_park[wib][0][lane], b = s_park[wib][1][lane], c = s_park[wib][2][lane];
-            oxy = pack2(a.x, a.y); oz = a.z; frac = a.w;
-            dxy = pack2(b.x, b.y); dz = b.z; steps = __float_as_int(b.w);
-            ivxy = pack2(c.x, c.y); ivz = c.z; fexit = c.w;
-            corner(b.x, b.y);
-        }
         // 2. idle lanes take rays
         assign(__ballot_sync(kFull, my < 0));
         if (!__any_sync(kFull, my >= 0)) {
             // nothing in flight and nothing set up: no task was left (a task of another world
             // would have been set up above, the lanes being drained)
-            if ((pending >= 0 || loaded > issued) && lane == 0) atomicOr(la.error, 1);
+            if ((pending >= 0 || taken < pooled) && lane == 0) atomicOr(la.error, 1);
             break;
         }
         // 3. march
-        const bool fast = ring_fast && __all_sync(kFull, fexit >= 0.0f || my < 0);
         if (mv.wide) {
-            if (fast) march(std::true_type{}, std::true_type{});
+            if (!slow) march(std::true_type{}, std::true_type{});
             else march(std::false_type{}, std::true_type{});
         } else {
-            if (fast) march(std::true_type{}, std::false_type{});
+            if (!slow) march(std::true_type{}, std::false_type{});
             else march(std::false_type{}, std::false_type{});
         }
     }
@@ -833,7 +825,7 @@ size_t stage_bytes(const WorldPass& w) {
     }
     if (w.n_compact <= 0) return 0;
     const size_t cg = (compact_cells(w.X, w.Y, w.Z) * (w.cgrid_wide ? 2 : 1) + 15) & ~(size_t)15;
-    const size_t bytes = kStageRingBytes + cg + (size_t)w.n_compact * 512;
+    const size_t bytes = kStagePoolBytes + cg + (size_t)w.n_compact * 512;
     return bytes <= (size_t)max_optin[dev] ? bytes : 0;
 }
 
