@@ -276,6 +276,7 @@ int DeviceWorld::sync_inputs(cudaStream_t stream) {
         if (fits) return LUMRAD_OK;
         grid_dirty = true;   // more than 256 ids: the whole world again, with uint16 compact ids
     }
+    if (!edited.empty()) grid_dirty = true;   // changed before a new palette: not on the device yet
     edited.clear();
     // a changed origin world or palette replaces the blockified frame (the next blockify rebuilds it)
     if (!h_cur.empty() && (grid_dirty || compact_dirty)) {

@@ -59,6 +59,23 @@ def test_edits_between_passes(types, frame):
             prev = _same(rw, grid, w, prev, k, frame)
 
 
+def test_edits_before_a_new_palette():
+    import lum_gb300
+    dims = (11, 8, 6)
+    w = worldgen.terrain_world(dims, seed=73, n_types=20)
+    grid = w.grid.copy()
+    with lum_gb300.RadianceWorld(dims, max_block_types=w.palette.shape[0]) as rw:
+        rw.load(w)
+        prev = random_prev(w)
+        rw.set_radiance(prev)
+        prev = _same(rw, grid, w, prev, 0, True)
+        for x, y, z, b in ((3, 3, 5, 9), (9, 1, 4, 4), (0, 7, 0, 0)):   # the first two above the terrain
+            rw.set_world_block(x, y, z, b)
+            grid[z, y, x] = b
+        rw.upload_block_palette()
+        _same(rw, grid, w, prev, 1, True)
+
+
 def test_edits_then_batch_and_server():
     import lum_gb300
     import oracle
