@@ -150,6 +150,8 @@ int check_batch_error(Batch* b) {
 int run_graph(Batch* b, int time_seed) {
     NvtxRange range("lumrad batch run");
     int rc;
+    for (auto& bw : b->worlds)
+        if ((rc = bw.ctx->world.wait_inputs(bw.ctx->stream))) return rc;
     if (b->dirty && (rc = build(b))) return rc;
     const int k = (int)(b->runs & 1);
     if (b->run_pending[k]) {   // the table of run - 2 may still be in flight

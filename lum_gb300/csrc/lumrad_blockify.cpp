@@ -231,6 +231,7 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
                                    c->stream));
     w.pal_dirty_end = used_end;
     w.uploads++;
+    w.unwaited = true;
     if (n_copies > 0) {
         int2* dev = nullptr;
         LUMRAD_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev), copies, 0));

@@ -262,8 +262,16 @@ int DeviceWorld::apply_cells(const uint32_t* idx, size_t n, const int16_t* g, bo
     CellEdit* dev = nullptr;
     LUMRAD_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev), h_cells[h], 0));
     LUMRAD_TRY(launch_apply_cells(dev, (int)n, d_grid, d_cgrid, cgrid_wide, X, Y, stream));
+    unwaited = true;
     LUMRAD_TRY(cudaEventRecord(ev_cells[h], stream));
     cells_half ^= 1;
+    return LUMRAD_OK;
+}
+
+int DeviceWorld::wait_inputs(cudaStream_t stream) {
+    if (!unwaited) return LUMRAD_OK;
+    LUMRAD_TRY(cudaStreamSynchronize(stream));
+    unwaited = false;
     return LUMRAD_OK;
 }
 

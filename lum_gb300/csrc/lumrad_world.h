@@ -107,6 +107,9 @@ struct DeviceWorld {
     size_t cells_cap[2] = {0, 0};
     cudaEvent_t ev_cells[2] = {nullptr, nullptr};
     int cells_half = 0;
+    // grid, masks or palette changed by kernels of the context's stream that nothing waited for:
+    // work on another stream waits first
+    bool unwaited = false;
     // one past the highest palette slot that may hold non-zero voxels on the device (blockify
     // clears the temporary slots up to here); every slot after a palette upload
     int pal_dirty_end = 1 << 30;
@@ -131,6 +134,7 @@ struct DeviceWorld {
     // Device bytes this world holds.
     size_t footprint() const;
     int sync_inputs(cudaStream_t stream);
+    int wait_inputs(cudaStream_t stream);   // until those kernels (of the context's stream) have ended
     // The n blocks at idx (repeats allowed) into the device's grid and compact grid, with their ids of
     // g; ids new to the world get compact ids, their slots uploaded, and with host_bits their masks
     // from the host palette.  *fits false: one of them needs a wider compact grid, nothing launched.

@@ -153,3 +153,32 @@ def test_models_frame_after_frame(n_slots):
             rw.update_radiance(_params(k))
             prev, _, _ = oracle.radiance_pass(fw, oracle.update_list(fw), prev=prev, rays=32, max_dist=96.0, blend=0.3, time_seed=k)
             assert rw.get_radiance().tobytes() == prev.tobytes()
+
+
+def test_models_then_batch():
+    """A batch runs on its own stream, right after the models' call returned."""
+    import lum_gb300
+    import oracle
+    w = worldgen.terrain_world((13, 11, 6), seed=74, n_types=20)
+    static, n_slots = w.palette.shape[0], 700
+    model = np.full((30, 24, 28), 77, np.uint8)
+    req = worldgen.all_probes(w.dims)
+    p = dict(rays=32, max_dist=96.0, blend=0.3)
+    with lum_gb300.RadianceWorld(w.dims, max_block_types=n_slots) as rw:
+        rw.load(w)
+        rw.load_model(model)
+        prev = random_prev(w)
+        rw.set_radiance(prev)
+        with lum_gb300.RadianceBatch([rw]) as b:
+            for k in range(3):
+                meshes = [(0, (1.0, 0.0, 0.0, 0.0), (16.0 * i + 3.0 * k, 40.0, 30.0)) for i in range(8)]
+                b.set_requests(0, req, lum_gb300.pass_params(**p))
+                rw.blockify(static, meshes)
+                b.run(k)
+                pal = np.zeros((n_slots, 16, 16, 16), np.uint8)
+                pal[:static] = w.palette
+                grid, pal = oracle.blockify(w.grid, pal, static, [model], meshes)
+                fw = worldgen.World(grid=grid, palette=pal, materials=w.materials)
+                prev, _, _ = oracle.radiance_pass(fw, req, prev=prev, time_seed=k, **p)
+                b.synchronize()
+                assert rw.get_radiance().tobytes() == prev.tobytes()
