@@ -621,13 +621,16 @@ __device__ __noinline__ uint32_t finalize_general(const WorldPass& w, const RayB
 }
 
 // Warps per CTA, and CTAs per SM of the lean and the general form.  The kernel waits on its chain of
-// dependent lookups and its barriers, so small CTAs pay: two warps for a group's eight tasks, 24 CTAs
-// per SM at 40 registers (44 B of spills).  On the demo's 8-pass step / a 64-ray demo frame / 64
-// worlds batched: 717 / 186 / 2,601 us; four warps 730 / 191 / 2,700; eight warps, one task each,
-// 725 / 197 / 2,775; two warps at 32 registers 836 / 196 / 2,649, at 48 registers 754 / 190 / 2,627;
-// one warp 793 / 190 / 2,648.
+// dependent lookups and its barriers, so small CTAs pay: two warps for a group's eight tasks.  Of the
+// SM's 256 KB their shared memory (3.4 + 1 KB a CTA) leaves the L1 less the more of them run, and the
+// L1 (45% hits; 8 KB of rays a CTA, the world, the taps) decides: 21 CTAs fit 100 KB, at 48 registers.
+// On the demo's 8-pass step / a 64-ray demo frame / 64 worlds batched: 673 / 166.5 / 2,188 us (with 24
+// CTAs at 40 registers, of which 22 ran, 688 / 170.7 / 2,203; 18: 722 / 175.6 / 2,245; 16: 724 / 180 /
+// 2,265; 132 KB of shared memory for all 24: 725 / 174 / 2,247).  Before these lines, at 717 / 186 /
+// 2,601: four warps 730 / 191 / 2,700; eight warps, one task each, 725 / 197 / 2,775; one warp 793 / 190 /
+// 2,648.
 constexpr int kFinCtaWarps = 2;
-constexpr int kFinLeanCtas = 24, kFinGeneralCtas = 16;
+constexpr int kFinLeanCtas = 21, kFinGeneralCtas = 16;
 // A launch of at most this many groups per SM has no second round of CTAs to keep the SMs busy: it
 // runs a warp per task (6 CTAs per SM), whose CTAs finish sooner.  One 64-ray pass of 79 / 306 / 832 /
 // 1,728 / 2,693 / 4,224 groups on 152 SMs: 20.7 / 25.6 / 31.0 / 44.7 / 55.5 / 73.7 us against 20.8 /
@@ -635,6 +638,7 @@ constexpr int kFinLeanCtas = 24, kFinGeneralCtas = 16;
 // The general form's warp-per-task CTAs run 4 to an SM: an R = 96 pass of 459 groups 28.6 against 32.8
 // us, of 1,570 groups 92.6 against 86.0.
 constexpr int kFinFewGroups = 16, kFinFewGeneral = 4;
+constexpr int kFinFewLeanCtas = 6, kFinFewGeneralCtas = 4;
 
 // One group of eight consecutive tasks (one CTA's work).  A warp per task in lock step had 20 of 32
 // lanes active: odd rays of a subgroup point the other way, so most tasks mix hits and misses.  Here
@@ -689,15 +693,17 @@ __device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, 
     }
     __syncthreads();
     // 2. the hits, packed 32 to a warp (the first 32 to another warp in each group, so that every
-    // scheduler of the SM gets its share)
+    // scheduler of the SM gets its share).  Their rays leave the L1 with this read: keeping them costs the
+    // 8-pass step 0.6%, not reading the hits' in step 1 1.4%.  (The general form's 16 CTAs leave the L1
+    // larger: there an R = 96 pass takes 71.7 us with them kept, 73.2 without.)
     const int n_hits = sh.n_hits;
 #pragma unroll 1
     for (int j = (int)(threadIdx.x + 32 * (group % CW)) % (32 * CW); !RECORD && j < n_hits; j += 32 * CW) {
         const int ray = sh.hit[j], idx = first + ray;
         const uint2 res = la.rays.res[idx];
         if (!(res.y & kInfoRegular)) continue;   // below
-        const float4 od = la.rays.od[idx];
-        const float2 dd = la.rays.dd[idx];
+        const float4 od = IN_CTA ? load_last(la.rays.od + idx) : la.rays.od[idx];
+        const float2 dd = IN_CTA ? load_last(la.rays.dd + idx) : la.rays.dd[idx];
         const float3 o = make_float3(od.x, od.y, od.z), d = make_float3(od.w, dd.x, dd.y);
         const float frac = __uint_as_float(res.x);
         float3 u;
@@ -760,7 +766,8 @@ __device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, 
 // PERSIST (launches sized on the device): a fixed grid walks the 8-task groups of the device's
 // task count; otherwise one CTA per group.
 template <class Store, bool RECORD, bool IN_CTA, bool PERSIST = false, bool SINGLE = false, int CW = kFinCtaWarps>
-__global__ void __launch_bounds__(CW * 32, (IN_CTA ? kFinLeanCtas : kFinGeneralCtas) * kFinCtaWarps / CW)
+__global__ void __launch_bounds__(CW * 32, CW == kFinCtaWarps ? (IN_CTA ? kFinLeanCtas : kFinGeneralCtas)
+                                              : (IN_CTA ? kFinFewLeanCtas : kFinFewGeneralCtas))
 finalize_kernel(const __grid_constant__ LaunchArgs la) {
     if (la.after_march) grid_dependency_wait();
     grid_launch_dependents();   // the next pass's launch may start its volume-free part
