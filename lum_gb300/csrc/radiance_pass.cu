@@ -185,9 +185,9 @@ __device__ __noinline__ long long refill_block(const LaunchArgs& la, int n_round
 }
 
 // What bounds it: instruction issue (84% of the slots on the demo's 8-pass launch, every world
-// lookup in shared memory).  Per 32-ray task that launch issues 897 warp instructions, of which the
+// lookup in shared memory).  Per 32-ray task that launch issues 890 warp instructions, of which the
 // set-up with its first step is about 400 and an iteration (3 steps of about 45 and the hand-out)
-// 200.  The launch: 436 -> 371 us, 452 -> 376 M warp instructions, with: lookups without range
+// 200.  The launch: 436 -> 366 us, 452 -> 373 M warp instructions, with: lookups without range
 // tests or conversions for regular rays (solid_inside), x and y in register pairs, the first step
 // in the set-up, results and hand-outs once per three steps, and reciprocals and the square root
 // without their checks for operands that cannot occur.  The set-up's x and y in register pairs too: the
@@ -667,28 +667,43 @@ __device__ __forceinline__ void finalize_group(const LaunchArgs& la, int group, 
         n_tasks = min(n_tasks, (long long)(__ldcg(la.dev_count) / wp->size) * (wp->R >> 5));
     const int first = (t0 - la.ray_origin) * kTaskRays;   // the group's first ray in the ray buffer
     // 1. the tasks' rays, one warp a task: the hits into the CTA's list, the misses' light.  (Every
-    // ray is read here, through L1: a hit's origin and direction then wait there for step 2.)
+    // ray is read here, through L1: a hit's origin and direction then wait there for step 2.  Two
+    // tasks' loads at a time: every probe of 64x64x32 / 64 worlds batched / a 64-ray demo frame 1,741 / 2,214 /
+    // 167.4 -> 1,735 / 2,198 / 167.0 us; four at a time 0.6% slower than two.)
     unsigned lookups = 0;
+    constexpr int kBatch = CW < kFinWarps ? 2 : 1;   // tasks whose rays a warp reads before it uses them
 #pragma unroll
-    for (int k = w; k < kFinWarps; k += CW) {
-        if (t0_local + k >= n_tasks) break;
-        const int idx = first + k * kTaskRays + lane;
-        const uint2 res = la.rays.res[idx];
-        const float2 dd = la.rays.dd[idx];
-        const float4 od = la.rays.od[idx];
-        const bool hit = res.y & kInfoHit;
-        lookups += res.y & 0xffffu;
-        const unsigned hm = __ballot_sync(kFull, hit);
-        int base = 0;
-        if (lane == 0 && hm) base = atomicAdd(&sh.n_hits, __popc(hm));
-        base = __shfl_sync(kFull, base, 0);
-        if (hit) {
-            sh.hit[base + __popc(hm & ((1u << lane) - 1u))] = (uint8_t)(k * kTaskRays + lane);
-            if (!(res.y & kInfoRegular)) sh.irregular = 1;
-        } else {
-            sh.put_light(k, lane, sky_light(make_float3(od.w, dd.x, dd.y)));
-            if (RECORD)
-                record_miss(*wp, __uint_as_float(res.x), res.y, __ldcg(la.ray_blk + idx), (long long)(t0_local + k) * kTaskRays + lane);
+    for (int k0 = w; k0 < kFinWarps; k0 += kBatch * CW) {
+        uint2 res[kBatch];
+        float2 dd[kBatch];
+        float4 od[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+            const int k = k0 + u * CW, idx = first + k * kTaskRays + lane;
+            if (t0_local + k >= n_tasks) break;
+            res[u] = la.rays.res[idx];
+            dd[u] = la.rays.dd[idx];
+            od[u] = la.rays.od[idx];
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+            const int k = k0 + u * CW;
+            if (t0_local + k >= n_tasks) break;
+            const bool hit = res[u].y & kInfoHit;
+            lookups += res[u].y & 0xffffu;
+            const unsigned hm = __ballot_sync(kFull, hit);
+            int base = 0;
+            if (lane == 0 && hm) base = atomicAdd(&sh.n_hits, __popc(hm));
+            base = __shfl_sync(kFull, base, 0);
+            if (hit) {
+                sh.hit[base + __popc(hm & ((1u << lane) - 1u))] = (uint8_t)(k * kTaskRays + lane);
+                if (!(res[u].y & kInfoRegular)) sh.irregular = 1;
+            } else {
+                sh.put_light(k, lane, sky_light(make_float3(od[u].w, dd[u].x, dd[u].y)));
+                if (RECORD)
+                    record_miss(*wp, __uint_as_float(res[u].x), res[u].y, __ldcg(la.ray_blk + first + k * kTaskRays + lane),
+                                (long long)(t0_local + k) * kTaskRays + lane);
+            }
         }
     }
     __syncthreads();
