@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "lumrad.h"
+#include "lumrad_cells.h"
 
 namespace lumrad {
 
@@ -50,11 +51,6 @@ inline RayBuffer ray_buffer(void* base, size_t cap) {
     return RayBuffer{reinterpret_cast<float4*>(p), reinterpret_cast<float2*>(p + 16 * cap),
                      reinterpret_cast<uint2*>(p + 24 * cap)};
 }
-
-// Cells of a world's compact grid: one more than the grid on the high side of each axis, all of
-// block 0 (what a lookup past the grid reads), so that the march reads the cell a ray leaves the
-// world through without testing the grid's range.
-inline size_t compact_cells(int X, int Y, int Z) { return (size_t)(X + 1) * (Y + 1) * (Z + 1); }
 
 // One world's pass as the kernels see it (all pointers are device pointers).
 //
