@@ -127,7 +127,8 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
 
     // blockify (host): temporary slots from static_blocks up, in mesh order, over the origin world:
     // the last frame's blocks get their origin ids again, this frame's are listed
-    if (w.h_cur.empty()) w.h_cur = w.h_grid;
+    const bool had_frame = !w.h_cur.empty();
+    if (!had_frame) w.h_cur = w.h_grid;
     int16_t* cur = w.h_cur.data();
     std::vector<std::pair<uint32_t, int16_t>> last;   // the last frame's ids, put back if this one fails
     std::vector<uint32_t> cells = w.blk_cells;        // the last frame's blocks, then this one's
@@ -138,6 +139,10 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
     }
     const size_t first_new = cells.size();
     auto undo = [&](int code) {
+        if (!had_frame) {
+            w.h_cur.clear();
+            return code;
+        }
         for (size_t k = first_new; k < cells.size(); k++) cur[cells[k]] = w.h_grid[cells[k]];
         for (const auto& e : last) cur[e.first] = e.second;
         return code;
