@@ -121,8 +121,8 @@ list_scan_kernel(const int* __restrict__ counts, int n, int* __restrict__ offset
 // kBitsCtas), of the bits before its own; the last CTA then also writes the length.
 constexpr int kDirectCtas = 4096, kBitsCtas = 1024;
 __global__ void __launch_bounds__(kListCta)
-list_write_kernel(const uint32_t* __restrict__ bits, const int* __restrict__ counts, const int* __restrict__ offsets, int X,
-                  int Y, unsigned W, short4* __restrict__ out, int* __restrict__ total, int* __restrict__ total2) {
+list_write_kernel(const uint32_t* bits, const int* counts, const int* offsets, int X, int Y, unsigned W, short4* out, int* total,
+                  int* total2) {
     grid_launch_dependents();
     __shared__ int s_pre[kListCta / 32], s_sum[kListCta / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -275,7 +275,7 @@ list_specials_kernel(const short4* __restrict__ sp, int ns, const uint32_t* __re
 }
 
 template <typename V>
-__global__ void shift_kernel(const V* __restrict__ src, V* __restrict__ dst, int X, int Y, int Z, int sx, int sy,
+__global__ void shift_kernel(const V* src, V* dst, int X, int Y, int Z, int sx, int sy,
                              int sz, long long W) {
     grid_launch_dependents();
     grid_dependency_wait();
@@ -348,7 +348,7 @@ __device__ __noinline__ float3 gather_general(const typename Store::T* rad, int 
 // [0, 1], on which the [0, 2] clamp does nothing.  Squares and distances are kept negated, so that
 // each residual is one paired FMA.
 template <class Store>
-__device__ __forceinline__ float3 gather_point(const typename Store::T* __restrict__ rad, int X, int Y, int Z, float px,
+__device__ __forceinline__ float3 gather_point(const typename Store::T* rad, int X, int Y, int Z, float px,
                                                float py, float pz, float nx, float ny, float nz) {
     const int zx = min(max(__float2int_rd(fsub(px, 8.0f)), 0) >> 4, X);
     const int zy = min(max(__float2int_rd(fsub(py, 8.0f)), 0) >> 4, Y);
@@ -432,8 +432,7 @@ __device__ __forceinline__ float3 gather_point(const typename Store::T* __restri
 constexpr int kGatherCta = 256;
 template <class Store, class V>
 __global__ void __launch_bounds__(kGatherCta)
-gather_kernel(const typename Store::T* __restrict__ rad, int X, int Y, int Z, const float* __restrict__ pts, int n,
-              float* __restrict__ out) {
+gather_kernel(const typename Store::T* rad, int X, int Y, int Z, const float* pts, int n, float* out) {
     __shared__ __align__(16) float s_buf[6 * kGatherCta];
     grid_launch_dependents();
     grid_dependency_wait();
@@ -575,8 +574,7 @@ __global__ void __launch_bounds__(128) compact_bits_kernel(const uint8_t* __rest
 constexpr int kPackCta = 256;
 template <class Store, class V>
 __global__ void __launch_bounds__(kPackCta)
-pack_rgb_kernel(const typename Store::T* __restrict__ rad, float* __restrict__ out, long long W, const int* __restrict__ err,
-                int* __restrict__ err_out) {
+pack_rgb_kernel(const typename Store::T* rad, float* out, long long W, const int* err, int* err_out) {
     __shared__ __align__(16) float s_buf[3 * kPackCta];
     constexpr int kW = sizeof(V) / sizeof(float);
     grid_dependency_wait();

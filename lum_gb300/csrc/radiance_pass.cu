@@ -204,7 +204,7 @@ march_kernel(const __grid_constant__ LaunchArgs la) {
         for (int i = 0; i < la.n_worlds; i++) {
             const WorldPass& w = la.worlds[i];
             for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < w.n_groups; g += stride) {
-                const short4 q = __ldg(w.req + (g * w.size + w.shift));
+                const short4 q = w.req[g * w.size + w.shift];
                 if (q.x < 0 || q.y < 0 || q.z < 0 || q.x >= w.X || q.y >= w.Y || q.z >= w.Z) continue;
                 atomicOr(la.pass_mask + (q.x + (long long)w.X * (q.y + (long long)w.Y * q.z)), 1u << i);
             }
