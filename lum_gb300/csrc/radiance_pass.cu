@@ -637,6 +637,10 @@ constexpr int kFinLeanCtas = 21, kFinGeneralCtas = 16;
 // 32.4 / 36.8 / 46.5 / 55.4 / 73.5 us with two warps; the lines cross near 2,500.
 // The general form's warp-per-task CTAs run 4 to an SM: an R = 96 pass of 459 groups 28.6 against 32.8
 // us, of 1,570 groups 92.6 against 86.0.
+// Passes with hit records take it up to 16 groups per SM in both forms.  Their kernels, 64 rays over every
+// probe of 8x8x8 (128 groups) / 2% of 64x64x16 (164): 36.8 / 46.2 us with two warps, 24.2 / 32.0; 96 rays
+// over 20x20x8 (1,200) 60.7, 53.9; 64 rays over 20% of 64x64x16 (1,640) 92, 89; past the line two warps
+// do as without records (96 rays, 20% of 64x64x16, 4,915 groups, 110 us; a warp per task 165).
 constexpr int kFinFewGroups = 16, kFinFewGeneral = 4;
 constexpr int kFinFewLeanCtas = 6, kFinFewGeneralCtas = 4;
 
@@ -898,14 +902,17 @@ void launch_finalize(const LaunchArgs& args, int n, bool in_cta, cudaStream_t st
     const int groups = (n + kFinWarps - 1) / kFinWarps;
     const int blocks = groups + (args.pass_mask ? args.fin_copy : 0);
     if (blocks <= 0) return;
-    if (!RECORD && few_groups(n, in_cta, num_sms)) {
-        auto k = single ? (in_cta ? finalize_kernel<Store, false, true, false, true, kFinWarps> : finalize_kernel<Store, false, false, false, true, kFinWarps>)
-                        : (in_cta ? finalize_kernel<Store, false, true, false, false, kFinWarps> : finalize_kernel<Store, false, false, false, false, kFinWarps>);
-        launch_kernel(k, blocks, kFinWarps * 32, 0, stream, overlap, args);
+    auto pick = [&](auto warps) {   // (hit records are of one world)
+        constexpr int CW = decltype(warps)::value;
+        if (RECORD || single)
+            return in_cta ? finalize_kernel<Store, RECORD, true, false, true, CW> : finalize_kernel<Store, RECORD, false, false, true, CW>;
+        return in_cta ? finalize_kernel<Store, false, true, false, false, CW> : finalize_kernel<Store, false, false, false, false, CW>;
+    };
+    if (few_groups(n, in_cta || RECORD, num_sms)) {
+        launch_kernel(pick(std::integral_constant<int, kFinWarps>{}), blocks, kFinWarps * 32, 0, stream, overlap, args);
         return;
     }
-    auto k = single ? (in_cta ? finalize_kernel<Store, RECORD, true, false, true> : finalize_kernel<Store, RECORD, false, false, true>)
-                    : (in_cta ? finalize_kernel<Store, RECORD, true> : finalize_kernel<Store, RECORD, false>);
+    auto k = pick(std::integral_constant<int, kFinCtaWarps>{});
     launch_kernel(k, blocks, kFinCtaWarps * 32, 0, stream, overlap, args);
 }
 
