@@ -1125,23 +1125,31 @@ namespace lumrad {
 namespace {
 
 constexpr int kNoAllocMaxBlocks = LUMRAD_NOALLOC_MAX_BLOCKS;
-constexpr int kNoAllocRoundTasks = 3840;
+// The most tasks of a round: 4,096, as many as the array holds beside the compact grid (noalloc_round_tasks).  (At
+// 3,840, beside room for the largest grid of all, a pass of 4,096 tasks took two rounds: 16x16x8 blocks, 64
+// rays, 70.2 us a call; one round, and its finalize with a warp per task, 44.2.)
+constexpr int kNoAllocRoundTasks = 4096;
 // the most cells of a compact grid of kNoAllocMaxBlocks blocks (compact_cells): a world of one
 // block's height, 2047 blocks long
 constexpr size_t kNoAllocMaxCells = 2 * ((size_t)kNoAllocMaxBlocks + 2047 + kNoAllocMaxBlocks / 2047 + 1);
 constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 // byte offsets of the parts of the array
-constexpr size_t kNaCgrid = 0;                                                        // uint16 per cell
-constexpr size_t kNaCbits = align256(kNaCgrid + 2 * kNoAllocMaxCells);                 // 512 B per compact id
-constexpr size_t kNaRays = align256(kNaCbits + (size_t)(LUMRAD_MAX_BLOCK_SLOTS + 2) * 512);
+constexpr size_t kNaCbits = 0;                                                        // 512 B per compact id
 // the direction tables for R = 32, 64, 128, 256 back to back (480 entries), uploaded once per device
-constexpr size_t kNaDirs = align256(kNaRays + (size_t)kNoAllocRoundTasks * kTaskRays * kRayBytes);
+constexpr size_t kNaDirs = align256(kNaCbits + (size_t)(LUMRAD_MAX_BLOCK_SLOTS + 2) * 512);
 constexpr int kNaDirEntries = 32 + 64 + 128 + 256;
 constexpr size_t kNaQueue = align256(kNaDirs + kNaDirEntries * sizeof(float4));
 constexpr size_t kNaError = kNaQueue + kQueueWords * sizeof(unsigned long long);
 constexpr size_t kNaStats = align256(kNaError + sizeof(int));
-constexpr size_t kNaBytes = align256(kNaStats + 2 * sizeof(unsigned long long));
-static_assert(kNaBytes <= (8u << 20), "no-allocation scratch must stay under 8 MiB");
+constexpr size_t kNaCgrid = align256(kNaStats + 2 * sizeof(unsigned long long));     // uint16 per cell, then the rays
+constexpr size_t kNaBytes = 8u << 20;
+// Tasks of a round over a world of `cells` compact-grid cells: a multiple of 8 (a probe's subgroups share a
+// CTA of the finalize).
+constexpr int noalloc_round_tasks(size_t cells) {
+    const size_t room = (kNaBytes - align256(kNaCgrid + 2 * cells)) / (kTaskRays * kRayBytes) / kFinWarps * kFinWarps;
+    return room < (size_t)kNoAllocRoundTasks ? (int)room : kNoAllocRoundTasks;
+}
+static_assert(noalloc_round_tasks(kNoAllocMaxCells) >= 4000, "rounds as long beside any grid");
 
 }  // namespace
 }  // namespace lumrad
@@ -1315,17 +1323,21 @@ extern "C" int lumrad_radiance_pass_noalloc(const int* world_size, const int16_t
     la.n_tasks = n_tasks;
     la.queue = queue;
     la.error = error;
-    la.rays = ray_buffer(base + kNaRays, (size_t)kNoAllocRoundTasks * kTaskRays);
-    const int blocks = march_grid(false, nd->num_sms, std::min<long long>(n_tasks, kNoAllocRoundTasks));
+    const size_t cells = compact_cells(w.X, w.Y, w.Z);
+    const int round = noalloc_round_tasks(cells);
+    la.rays = ray_buffer(base + align256(kNaCgrid + 2 * cells), (size_t)round * kTaskRays);
+    const int blocks = march_grid(false, nd->num_sms, std::min<long long>(n_tasks, round));
     la.total_warps = blocks * kWarps;
-    for (long long c0 = 0; c0 < n_tasks; c0 += kNoAllocRoundTasks) {
+    for (long long c0 = 0; c0 < n_tasks; c0 += round) {
         la.chunk_begin = (int)c0;
-        la.chunk_end = (int)std::min(c0 + (long long)kNoAllocRoundTasks, n_tasks);
+        la.chunk_end = (int)std::min(c0 + (long long)round, n_tasks);
         la.ray_origin = la.chunk_begin;
         const int tasks = la.chunk_end - la.chunk_begin;
         if (tasks < kCtaQueueTasksPerWarp * la.total_warps) march_kernel<false, false, true><<<blocks, kWarps * 32, 0, stream>>>(la);
         else march_kernel<false><<<blocks, kWarps * 32, 0, stream>>>(la);
-        finalize_kernel<StoreF32, false, true, false, true><<<(tasks + kFinWarps - 1) / kFinWarps, kFinCtaWarps * 32, 0, stream>>>(la);
+        // (a round has few groups: kFinFewGroups)
+        finalize_kernel<StoreF32, false, true, false, true, kFinWarps>
+            <<<(tasks + kFinWarps - 1) / kFinWarps, kFinWarps * 32, 0, stream>>>(la);
     }
     LUMRAD_TRY(cudaGetLastError());
     return LUMRAD_OK;
