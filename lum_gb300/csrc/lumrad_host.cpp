@@ -1163,7 +1163,7 @@ int lumrad_build_dirty_list(LumRadContext ctx, const LumRadEdit* edits, int n_ed
     LUMRAD_TRY(cudaSetDevice(c->device));
     int rc = c->ensure_list_scratch();
     if (rc) return rc;
-    if (dirty_rows_fit((long long)w.W, n_edits, radius)) {
+    if (dirty_rows_fit(w.X, w.Y, w.Z, n_edits, radius)) {
         // edits read from, list and length written to page-locked memory: no copies, one wait
         if ((rc = c->ensure_list_staging((size_t)n_edits))) return rc;
         if (n_edits > 0) std::memcpy(c->h_list + w.W, edits, (size_t)n_edits * sizeof(short4));

@@ -217,7 +217,7 @@ cudaError_t launch_dirty_list(const short4* edits, int n_edits, int X, int Y, in
 
 // The same for a few edits (dirty_rows_fit), without masks: bits are the list scratch's; edits and out
 // may be page-locked host memory's device addresses.
-bool dirty_rows_fit(long long W, int n_edits, int radius);
+bool dirty_rows_fit(int X, int Y, int Z, int n_edits, int radius);
 cudaError_t launch_dirty_rows(const short4* edits, int n_edits, int X, int Y, int Z, int radius, uint32_t* bits, short4* out,
                               int* count, cudaStream_t stream);
 

@@ -174,19 +174,18 @@ cudaError_t launch_list_write(const ListScratch& s, int X, int Y, long long W, s
                          (unsigned)W, out, nullptr, nullptr);
 }
 
-// Dirty probes of a few edits (Chebyshev distance <= r): each row of an edit's cube sets its run of
-// bits, a thread per row; the list is then written from the bits.  A memset and two launches,
-// where the dilation below takes a memset and five: used while the rows are at most 2^21 and the
-// world at most 262,144 blocks.
+// Dirty probes of a few edits (Chebyshev distance <= r): each row of an edit's cube inside the world sets
+// its run of bits, a thread per row; the list is then written from the bits.  A memset and two launches,
+// where the dilation below takes a memset and five: used where dirty_rows_fit says.
 __global__ void dirty_rows_kernel(const short4* __restrict__ edits, int rows, int X, int Y, int Z, int r,
                                   uint32_t* __restrict__ bits) {
     grid_launch_dependents();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= rows) return;
-    const int side = 2 * r + 1, row = k % (side * side);
-    const short4 e = edits[k / (side * side)];
-    const int y = e.y + row % side - r, z = e.z + row / side - r;
-    if (y < 0 || y >= Y || z < 0 || z >= Z) return;
+    const int ny = min(2 * r + 1, Y), nz = min(2 * r + 1, Z), row = k % (ny * nz);
+    const short4 e = edits[k / (ny * nz)];
+    const int y = max(e.y - r, 0) + row % ny, z = max(e.z - r, 0) + row / ny;
+    if (y > min(e.y + r, Y - 1) || z > min(e.z + r, Z - 1)) return;
     const int x0 = max(e.x - r, 0), x1 = min(e.x + r, X - 1);   // at most 31 blocks: two words
     const unsigned i0 = (unsigned)x0 + (unsigned)X * ((unsigned)y + (unsigned)Y * (unsigned)z), i1 = i0 + (unsigned)(x1 - x0);
     const uint32_t m0 = ~0u << (i0 & 31), m1 = ~0u >> (31 - (i1 & 31));
@@ -691,15 +690,25 @@ cudaError_t launch_dirty_list(const short4* edits, int n_edits, int X, int Y, in
     return launch_list_write(s, X, Y, W, out, count, nullptr, stream);
 }
 
-bool dirty_rows_fit(long long W, int n_edits, int radius) {
-    const long long side = 2LL * radius + 1;
-    return list_scratch_ctas(W) <= kBitsCtas && n_edits * side * side <= 1LL << 21;
+static long long dirty_rows(int n_edits, int Y, int Z, int radius) {
+    return (long long)n_edits * std::min(2 * radius + 1, Y) * std::min(2 * radius + 1, Z);
+}
+
+// The line between the rows of bits and the dilation, from calls of both (rows / dilation): the kernel reads the
+// edits from the host's memory (200,000 of them, radius 0, 16x16x8 blocks: 410 / 330 us, 4,096: 25 / 61), rows
+// close together wait for each other's words (8x8x8, 500,000 rows 115 / 85, 128,000 rows 29 / 55; 64x64x16,
+// 992,000 rows 69 / 78), and the list goes to the host's memory block by block (64x64x64, a list of
+// up to 262,144: 162 / 74, of 41,000: 40 / 89).  Neither form is slower than the dilation alone was.
+bool dirty_rows_fit(int X, int Y, int Z, int n_edits, int radius) {
+    const long long W = (long long)X * Y * Z, rows = dirty_rows(n_edits, Y, Z, radius);
+    return list_scratch_ctas(W) <= kBitsCtas && n_edits <= 4096 && rows <= std::min(std::max(32 * W, 1LL << 17), 1LL << 20) &&
+           std::min(W, rows * std::min(2 * radius + 1, X)) <= 1LL << 16;
 }
 
 cudaError_t launch_dirty_rows(const short4* edits, int n_edits, int X, int Y, int Z, int radius, uint32_t* bits, short4* out,
                               int* count, cudaStream_t stream) {
     const long long W = (long long)X * Y * Z;
-    const long long rows = (long long)n_edits * (2 * radius + 1) * (2 * radius + 1);
+    const long long rows = dirty_rows(n_edits, Y, Z, radius);
     cudaError_t e = cudaMemsetAsync(bits, 0, list_scratch_words(W) * sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     if (rows > 0) dirty_rows_kernel<<<(int)((rows + 255) / 256), 256, 0, stream>>>(edits, (int)rows, X, Y, Z, radius, bits);
