@@ -211,8 +211,11 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
     // the slots this frame writes: every id from static_blocks up present in the grid (made here
     // or set by the caller), below n_slots
     if (w.origin_end < 0) {
-        w.origin_end = 0;
-        for (size_t i = 0; i < w.W; i++) w.origin_end = std::max(w.origin_end, (int)w.h_grid[i] + 1);
+        w.origin_end = w.slot_end = 0;
+        for (size_t i = 0; i < w.W; i++) {
+            w.origin_end = std::max(w.origin_end, (int)w.h_grid[i] + 1);
+            w.slot_end = std::max(w.slot_end, w.slot_of(w.h_grid[i]) + 1);
+        }
     }
     const int used_end = std::min(std::max(std::max(counter, w.origin_end), static_blocks), w.n_slots);
     // the changed blocks into the device's grids; if an id needs a wider compact grid, the whole world
@@ -235,6 +238,7 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
         LUMRAD_TRY(cudaMemsetAsync(w.d_pal + (size_t)static_blocks * 4096, 0, (size_t)(clear_end - static_blocks) * 4096,
                                    c->stream));
     w.pal_dirty_end = used_end;
+    w.blk_static = std::min(w.blk_static, static_blocks);
     w.uploads++;
     w.unwaited = true;
     if (n_copies > 0) {

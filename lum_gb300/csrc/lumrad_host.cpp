@@ -125,6 +125,7 @@ int DeviceWorld::readmit(cudaStream_t stream) {
     LUMRAD_TRY(cudaMemcpyAsync(d_grid, h_grid.data(), W * sizeof(int16_t), cudaMemcpyHostToDevice, stream));
     LUMRAD_TRY(cudaMemcpyAsync(d_pal, h_pal_dev.data(), h_pal_dev.size(), cudaMemcpyHostToDevice, stream));
     pal_dirty_end = n_slots;
+    blk_static = 1 << 30;
     LUMRAD_TRY(cudaMemcpyAsync(d_mats, h_mats_dev.data(), LUMRAD_MATERIALS * sizeof(float4), cudaMemcpyHostToDevice,
                                stream));
     LUMRAD_TRY(cudaMemsetAsync(d_stats, 0, 2 * sizeof(unsigned long long), stream));
@@ -148,6 +149,7 @@ void DeviceWorld::build_compact(const int16_t* g, bool host_bits) {
     id_to_c[0] = 0;
     reps.push_back(0);
     n_compact = 1;
+    if (host_bits) frame_ids = false;
     h_cbits.assign(128, 0u);
     skip_host_bits = !host_bits;
     for (int k = 0; k < 4096 && n_slots > 0 && host_bits; k++)   // block 0 reads palette slot 0 like any other id
@@ -276,12 +278,23 @@ int DeviceWorld::wait_inputs(cudaStream_t stream) {
 }
 
 int DeviceWorld::sync_inputs(cudaStream_t stream) {
-    if (!grid_dirty && !compact_dirty && !edited.empty()) {
+    // a changed origin world replaces a frame of models: its blocks get their origin ids again with the
+    // edits, if the world's ids have slots that no frame has written, whose masks are right (an edit beside
+    // eight 32^3 models in 64x64x16 blocks, with the next models and the frame: 826 -> 310 us; the whole
+    // world uploaded and numbered again otherwise)
+    const bool masks_right = (h_cur.empty() && !frame_ids) || (slot_end >= 0 && slot_end <= blk_static);
+    if (!grid_dirty && !compact_dirty && !edited.empty() && masks_right) {
         bool fits = true;
+        edited.insert(edited.end(), blk_cells.begin(), blk_cells.end());
         const int rc = apply_cells(edited.data(), edited.size(), h_grid.data(), true, stream, &fits);
         if (rc) return rc;
         edited.clear();
-        if (fits) return LUMRAD_OK;
+        if (fits) {
+            frame_ids = frame_ids || !h_cur.empty();
+            h_cur.clear();
+            blk_cells.clear();
+            return LUMRAD_OK;
+        }
         grid_dirty = true;   // more than 256 ids: the whole world again, with uint16 compact ids
     }
     if (!edited.empty()) grid_dirty = true;   // changed before a new palette: not on the device yet
@@ -294,7 +307,7 @@ int DeviceWorld::sync_inputs(cudaStream_t stream) {
     }
     if (grid_dirty || compact_dirty) uploads++;
     if (grid_dirty) {
-        origin_end = -1;
+        origin_end = slot_end = -1;
         LUMRAD_TRY(cudaMemcpyAsync(d_grid, h_grid.data(), W * sizeof(int16_t), cudaMemcpyHostToDevice, stream));
         grid_dirty = false;
         compact_dirty = true;
@@ -962,9 +975,11 @@ int lumrad_set_world_block(LumRadContext ctx, int x, int y, int z, int16_t block
     const size_t idx = (size_t)x + (size_t)w.X * ((size_t)y + (size_t)w.Y * z);
     w.h_grid[idx] = block;
     if (w.origin_end >= 0) w.origin_end = std::max(w.origin_end, (int)block + 1);
-    // uploaded before the next pass, as exec_copies does every frame: block by block while they are
-    // few (an eighth of the world) and no blockified frame has to give way to the changed world
-    if (!w.grid_dirty && !w.compact_dirty && w.h_cur.empty() && w.edited.size() < w.W / 8 + 64) w.edited.push_back((uint32_t)idx);
+    if (w.slot_end >= 0) w.slot_end = std::max(w.slot_end, w.slot_of(block) + 1);
+    // uploaded before the next pass, as exec_copies does every frame: block by block while they are few (an
+    // eighth of the world: the pass after 8,192 edits of 64x64x16 blocks 84 us, 371 with the whole
+    // world uploaded and numbered again; after 65,536 of 128x128x32 557 and 945)
+    if (!w.grid_dirty && !w.compact_dirty && w.edited.size() < w.W / 8 + 64) w.edited.push_back((uint32_t)idx);
     else w.grid_dirty = true;
     return LUMRAD_OK;
 }
@@ -1001,6 +1016,7 @@ int lumrad_upload_block_palette(LumRadContext ctx) {
     w.h_pal_dev = w.h_pal;
     LUMRAD_TRY(cudaMemcpyAsync(w.d_pal, w.h_pal_dev.data(), w.h_pal_dev.size(), cudaMemcpyHostToDevice, c->stream));
     w.pal_dirty_end = w.n_slots;
+    w.blk_static = 1 << 30;
     LUMRAD_TRY(cudaStreamSynchronize(c->stream));
     w.compact_dirty = true;
     return LUMRAD_OK;

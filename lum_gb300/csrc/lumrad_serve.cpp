@@ -1023,8 +1023,8 @@ int lumrad_server_add_world(LumRadServer server, LumRadContext world, int* id) {
     DeviceWorld& dw = c->world;
     // a blockified frame is dropped: edits apply to the loaded world; and the upload is waited for (the
     // launches run on other streams)
-    if (!dw.h_cur.empty() || !dw.edited.empty()) dw.grid_dirty = true;
-    dw.origin_end = -1;   // the server's edits change the grid
+    if (!dw.h_cur.empty() || dw.frame_ids || !dw.edited.empty()) dw.grid_dirty = true;
+    dw.origin_end = dw.slot_end = -1;   // the server's edits change the grid
     int rc = dw.sync_inputs(c->stream);
     if (rc) return rc;
     if ((rc = prepare_world(dw, c->stream))) return rc;

@@ -97,7 +97,17 @@ struct DeviceWorld {
     // blockify: the frame's grid with temporary blocks (empty when not blockified)
     std::vector<int16_t> h_cur;
     std::vector<uint32_t> blk_cells;      // the blocks in which h_cur differs from h_grid
-    int origin_end = -1;                  // one past the highest block id of h_grid, or more (-1: not known)
+    // one past the highest block id of h_grid, and past the highest palette slot of its ids, or more
+    // (-1: not known)
+    int origin_end = -1, slot_end = -1;
+    // the lowest static_blocks of the models' frames since the palette's upload: below it the device's
+    // palette is the uploaded one
+    int blk_static = 1 << 30;
+    bool frame_ids = false;               // ids of a frame that left block by block keep their compact ids and masks
+    int slot_of(int16_t b) const {        // the palette slot of block id b, -1: none
+        const int slot = b >= 0 ? b : b + 64;
+        return b >= -63 && slot < n_slots ? slot : -1;
+    }
     // blocks of h_grid changed since its upload, while neither grid_dirty nor compact_dirty: applied
     // one by one (apply_cells) instead of uploading and renumbering the whole world
     std::vector<uint32_t> edited;
