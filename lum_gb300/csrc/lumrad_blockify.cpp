@@ -211,11 +211,18 @@ int lumrad_blockify(LumRadContext ctx, int static_blocks, const int* models, con
     // the slots this frame writes: every id from static_blocks up present in the grid (made here
     // or set by the caller), below n_slots
     if (w.origin_end < 0) {
-        w.origin_end = w.slot_end = 0;
+        // (plain maxima, which the compiler forms many at a time; a negative id's slot is at most the highest's)
+        const int16_t* g = w.h_grid.data();
+        const int n_slots = w.n_slots;
+        int top = -1, slot = -1, negative = -65;
         for (size_t i = 0; i < w.W; i++) {
-            w.origin_end = std::max(w.origin_end, (int)w.h_grid[i] + 1);
-            w.slot_end = std::max(w.slot_end, w.slot_of(w.h_grid[i]) + 1);
+            const int b = g[i];
+            top = std::max(top, b);
+            slot = std::max(slot, b < n_slots ? b : -1);
+            negative = std::max(negative, b < 0 && b >= -63 ? b : -65);
         }
+        w.origin_end = top + 1;
+        w.slot_end = std::max(slot, std::min(negative + 64, n_slots - 1)) + 1;
     }
     const int used_end = std::min(std::max(std::max(counter, w.origin_end), static_blocks), w.n_slots);
     // the changed blocks into the device's grids; if an id needs a wider compact grid, the whole world
