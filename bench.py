@@ -61,15 +61,15 @@ BATCH_ROUND_TASKS = 1 << 20   # 32-ray tasks per march/finalize round of a batch
 # DRAM bytes (read + write) of one step's kernels (the march launch over 8 passes and the 8
 # finalize launches, whose extra CTAs copy each pass's unlisted probes) in ncu captures of this
 # workload (the march's launch, and 3 of the 8 finalize launches scaled to 8); ncu replays with cold
-# caches (march 3.46 + 369.80 MB: most of the step's 430 MB of rays, 32 bytes each, leave the L2
-# before their finalize launches; finalizes 442.66 + 1.43 MB)
-NCU_DRAM_BYTES_PER_STEP = 817.35e6
-# L2 bytes (lts__t_bytes.sum) of the same launches in the same captures (march 881.1 MB: its world
-# lookups are shared-memory loads, finalizes 1581.3 MB)
-NCU_L2_BYTES_PER_STEP = 2462.4e6
+# caches (march 3.52 + 369.81 MB: most of the step's 430 MB of rays, 32 bytes each, leave the L2
+# before their finalize launches; finalizes 442.64 + 1.04 MB)
+NCU_DRAM_BYTES_PER_STEP = 817.0e6
+# L2 bytes (lts__t_bytes.sum) of the same launches in the same captures (march 881.6 MB: its world
+# lookups are shared-memory loads, finalizes 1585.5 MB)
+NCU_L2_BYTES_PER_STEP = 2467.1e6
 # Warp instructions (smsp__inst_executed.sum) of the same launches: the march over the 8 passes
-# (373.3 M) and the 8 finalize launches (200.1 M); deterministic up to the march queue's task order
-NCU_WARP_INST_PER_STEP = 373.3e6 + 200.1e6
+# (373.4 M) and the 8 finalize launches (202.4 M); deterministic up to the march queue's task order
+NCU_WARP_INST_PER_STEP = 373.4e6 + 202.4e6
 SCHEDULERS_PER_SM = 4
 
 

@@ -549,9 +549,9 @@ int Context::run_pass(const short4* d_reqs, int n, const LumRadPassParams* p_in,
     la.queue = d_queue;
     la.error = d_error;
     if ((rc = ensure_rays(la.n_tasks))) return rc;
-    // the march may start in the previous pass's finalize tail: see pass_mark (the list must not
-    // come from a kernel, the hits use the one record buffer)
-    // (over a device list it waits for the list's kernels before it reads anything of theirs)
+    // the march may start in the tail of the kernel before it: over a host list, of the previous pass's finalize
+    // (see pass_mark); over a list from kernels always, and it waits for them before it reads anything
+    // of theirs.  Not with hit records: they have one buffer
     const bool dependent = !p.record_hits && (dev_count || (pass_mark == api_calls - 1 && uploads_mark == world.uploads));
     la.rays = ray_buffer(d_rays[ray_side], ray_cap);
     ray_side ^= 1;

@@ -32,7 +32,8 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? l
 // The list kernels are bound by launch latency (a few us each, about 1 us of work at 65,536 blocks): two
 // launches instead of four, and the frame's kernels (scroll, list, march, finalize of few groups,
 // gather) each a programmatic dependent of the one before.  A lone 8x8x8 / 19x38x9 / 45x38x11 frame:
-// 39.6 / 57.2 / 81.2 -> 22.6 / 38.8 / 62.8 us.
+// 39.6 / 57.2 / 81.2 -> 22.6 / 38.8 / 62.8 us from call to result; among others (frames back to back) 8x8x8
+// 18.9 -> 13.4 us.
 //
 // The flags and counts (the grid does not come from a kernel: they are formed while the stream's
 // previous kernel still runs, then this one waits for it; see launch_kernel).
@@ -119,6 +120,10 @@ list_scan_kernel(const int* __restrict__ counts, int n, int* __restrict__ offset
 // The list from the bits.  A CTA's offset: offsets[blockIdx.x] of a scan of the counts; or, offsets
 // null (up to kDirectCtas CTAs), the sum of the counts before its own; or, both null (up to
 // kBitsCtas), of the bits before its own; the last CTA then also writes the length.
+// The lines: with the scan / the counts summed, the update list of 65,536 / 524,288 / 1,081,344 / 2,097,152 /
+// 4,194,304 blocks takes 27.8 / 31.3 / 41.0 / 64 / 98 and 17.3 / 26 / 38.6 / 53 / 100 us a call (the sums grow
+// with the square of the CTAs); the dirty list of 328 edits, by the dilation / from the bits, in
+// 262,144 / 524,288 / 1,048,576 / 2,097,152 blocks 66 / 70 / 82 / 106 and 39 / 44 / 56 / 98.
 constexpr int kDirectCtas = 4096, kBitsCtas = 1024;
 __global__ void __launch_bounds__(kListCta)
 list_write_kernel(const uint32_t* bits, const int* counts, const int* offsets, int X, int Y, unsigned W, short4* out, int* total,

@@ -184,7 +184,7 @@ __device__ __noinline__ long long refill_block(const LaunchArgs& la, int n_round
     return -1;
 }
 
-// What bounds it: instruction issue (84% of the slots on the demo's 8-pass launch, every world
+// What bounds it: instruction issue (83% of the slots on the demo's 8-pass launch, every world
 // lookup in shared memory).  Per 32-ray task that launch issues 890 warp instructions, of which the
 // set-up with its first step is about 400 and an iteration (3 steps of about 45 and the hand-out)
 // 200.  The launch: 436 -> 366 us, 452 -> 373 M warp instructions, with: lookups without range
@@ -623,9 +623,9 @@ __device__ __noinline__ uint32_t finalize_general(const WorldPass& w, const RayB
 // Warps per CTA, and CTAs per SM of the lean and the general form.  The kernel waits on its chain of
 // dependent lookups and its barriers, so small CTAs pay: two warps for a group's eight tasks.  Of the
 // SM's 256 KB their shared memory (3.4 + 1 KB a CTA) leaves the L1 less the more of them run, and the
-// L1 (45% hits; 8 KB of rays a CTA, the world, the taps) decides: 21 CTAs fit 100 KB, at 48 registers.
+// L1 (47% hits; 8 KB of rays a CTA, the world, the taps) decides: 21 CTAs, at 40 registers.
 // On the demo's 8-pass step / a 64-ray demo frame / 64 worlds batched: 673 / 166.5 / 2,188 us (with 24
-// CTAs at 40 registers, of which 22 ran, 688 / 170.7 / 2,203; 18: 722 / 175.6 / 2,245; 16: 724 / 180 /
+// CTAs, of which 22 ran, 688 / 170.7 / 2,203; 18: 722 / 175.6 / 2,245; 16: 724 / 180 /
 // 2,265; 132 KB of shared memory for all 24: 725 / 174 / 2,247).  Before these lines, at 717 / 186 /
 // 2,601: four warps 730 / 191 / 2,700; eight warps, one task each, 725 / 197 / 2,775; one warp 793 / 190 /
 // 2,648.
@@ -636,7 +636,8 @@ constexpr int kFinLeanCtas = 21, kFinGeneralCtas = 16;
 // 1,728 / 2,693 / 4,224 groups on 152 SMs: 20.7 / 25.6 / 31.0 / 44.7 / 55.5 / 73.7 us against 20.8 /
 // 32.4 / 36.8 / 46.5 / 55.4 / 73.5 us with two warps; the lines cross near 2,500.
 // The general form's warp-per-task CTAs run 4 to an SM: an R = 96 pass of 459 groups 28.6 against 32.8
-// us, of 1,570 groups 92.6 against 86.0.
+// us, of 1,570 groups 92.6 against 86.0.  Over a world table: a batch of one / two 8x8x8 worlds 47 / 49 us,
+// of 64 lists of 5% of such worlds 54, a served request 160, against 54 / 54.4, 61 and 171 with two warps.
 // Passes with hit records take it up to 16 groups per SM in both forms.  Their kernels, 64 rays over every
 // probe of 8x8x8 (128 groups) / 2% of 64x64x16 (164): 36.8 / 46.2 us with two warps, 24.2 / 32.0; 96 rays
 // over 20x20x8 (1,200) 60.7, 53.9; 64 rays over 20% of 64x64x16 (1,640) 92, 89; past the line two warps
@@ -648,7 +649,7 @@ constexpr int kFinFewLeanCtas = 6, kFinFewGeneralCtas = 4;
 // lanes active: odd rays of a subgroup point the other way, so most tasks mix hits and misses.  Here
 // the CTA's hits are refined and shaded 32 to a warp, and one lane per task and channel sums the
 // subgroup in the butterfly's order from shared memory: 38.3 -> 28.1 M warp instructions per pass of
-// the demo step.
+// the demo step when it was made, 25.3 M with the steps since.
 // IN_CTA: every probe of the launch combines inside one CTA (R/32 divides kFinWarps); the kernel
 // then has no global-memory combine.  SINGLE: the launch covers one world (a single pass, or one
 // pass of a several-pass call), read from the kernel's parameters, whose fields are operands from
